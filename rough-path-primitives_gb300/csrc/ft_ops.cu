@@ -382,11 +382,34 @@ constexpr size_t kStageLimit = 200 * 1024;
 
 }  // namespace
 
+// Whether the added term may be read element by element as the result is
+// written: it lies apart from the output, or is the output itself.
+template <typename T>
+static bool add_in_place(const Geometry& g, const TArg<T>& out, const TArg<T>& add, int64_t batch) {
+    if (!add.p || add.lo > add.hi || out.lo > out.hi) return true;
+    if (add.p == out.p && (batch == 1 || add.stride == out.stride)) return true;
+    auto begin = [&](const TArg<T>& t) { return t.p + g.db[t.lo]; };
+    auto end = [&](const TArg<T>& t) { return t.p + (batch - 1) * t.stride + g.db[std::min(t.hi, g.depth) + 1]; };
+    return end(add) <= begin(out) || end(out) <= begin(add);
+}
+
 template <typename T>
 cudaError_t launch_product(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ProductKind kind,
                            TArg<T> out, TArg<T> x, TArg<T> y, TArg<T> z, int64_t batch, double alpha,
                            double beta) {
     if (batch <= 0) return cudaSuccess;
+    if (column_product_fits<T>(g, dev)) {
+        TArg<T> add{nullptr, 0, 1, 0}, lhs = y, rhs = z;
+        switch (kind) {
+            case ProductKind::Fma: add = x; break;
+            case ProductKind::InplaceBCA: add = out; break;
+            case ProductKind::InplaceABC: add = z, lhs = out, rhs = y; break;
+            case ProductKind::InplaceBAC: add = z, rhs = out; break;
+            case ProductKind::InplaceMul: lhs = out, rhs = y; break;
+        }
+        if (add_in_place(g, out, add, batch))
+            return launch_column_product<T>(g, dev, s, out, add, lhs, rhs, batch, alpha, beta);
+    }
     const size_t smem_need = kBulkHeader + 3 * static_cast<size_t>(staged_elems<T>(g.dim)) * sizeof(T);
     const int staged = smem_need <= kStageLimit && smem_need <= static_cast<size_t>(dev.max_smem_optin);
     const size_t smem = staged ? smem_need : 0;

@@ -33,6 +33,13 @@ cudaError_t launch_product(const Geometry& g, const DeviceInfo& dev, cudaStream_
                            TArg<T> out, TArg<T> x, TArg<T> y, TArg<T> z, int64_t batch, double alpha,
                            double beta);
 
+// The column form of launch_product (widths 2..8, both factors in
+// shared memory) (ft_column.cu).
+template <typename T>
+bool column_product_fits(const Geometry& g, const DeviceInfo& dev);
+template <typename T>
+cudaError_t launch_column_product(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out, TArg<T> add,
+                                TArg<T> lhs, TArg<T> rhs, int64_t batch, double alpha, double beta);
 template <typename T>
 cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
                                 IntermediateKind kind, TArg<T> out, TArg<T> x, TArg<T> y,

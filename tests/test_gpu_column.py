@@ -1,0 +1,101 @@
+"""The compile-time-width per-operation kernels against plain numpy in FP64:
+products a column of coefficients at a time (csrc/ft_column.cu), at the edges of their tasks --
+levels shorter than a column's first letters, partial last groups of tensors,
+strided and unaligned rows, degree ranges, every in-place form."""
+import importlib
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+pkg = importlib.import_module("rough-path-primitives_gb300")
+
+EPS = {torch.float64: 2.0 ** -53, torch.float32: 2.0 ** -24}
+SHAPES = [(2, 2, 9), (2, 3, 613), (2, 7, 40), (3, 1, 5), (3, 2, 613), (3, 5, 40), (4, 3, 1300), (4, 4, 613),
+          (5, 2, 700), (5, 4, 33), (6, 3, 613), (7, 2, 33), (7, 4, 7), (8, 3, 330), (8, 1, 40), (6, 5, 3), (2, 12, 3)]
+
+
+def starts(W, D):
+    return np.concatenate([[0], np.cumsum([W ** n for n in range(D + 1)])])
+
+
+def restrict(x, W, D, r):
+    db, y = starts(W, D), np.zeros_like(x)
+    if r[0] <= min(r[1], D):
+        y[:, db[r[0]]:db[min(r[1], D) + 1]] = x[:, db[r[0]]:db[min(r[1], D) + 1]]
+    return y
+
+
+def product(x, y, W, D):
+    db, out = starts(W, D), np.zeros_like(x)
+    for n in range(D + 1):
+        for k in range(n + 1):
+            a, b = x[:, db[n - k]:db[n - k + 1]], y[:, db[k]:db[k + 1]]
+            out[:, db[n]:db[n + 1]] += (a[:, :, None] * b[:, None, :]).reshape(len(x), -1)
+    return out
+
+
+class Rows:
+    """A batch of tensors in a padded, offset buffer of sentinels."""
+
+    def __init__(self, rng, dtype, W, D, B, pad, offset, scale=1.0):
+        self.n, self.W, self.D, self.B = int(starts(W, D)[-1]), W, D, B
+        self.stride, self.offset = self.n + pad, offset
+        self.buf = torch.full((offset + B * self.stride,), 7.0, dtype=dtype, device="cuda")
+        self.rows = self.buf[offset:].view(B, self.stride)[:, :self.n]
+        self.rows.copy_(torch.from_numpy(rng.uniform(-scale, scale, (B, self.n))))
+
+    def host(self):
+        return self.rows.double().cpu().numpy()
+
+    def view(self, lo=0, hi=None):
+        return pkg.make_tensor_batch(self.buf, self.stride, lo, self.D if hi is None else hi, self.offset)
+
+
+def check(got, before, want, W, D, r, tol):
+    """`want` on the degrees r of the output, the old values elsewhere."""
+    db = starts(W, D)
+    lo, hi = db[r[0]], db[min(r[1], D) + 1]
+    assert np.array_equal(got[:, :lo], before[:, :lo]) and np.array_equal(got[:, hi:], before[:, hi:])
+    err = np.max(np.abs(got - want)[:, lo:hi])
+    assert err <= tol, f"{err:.3e} > {tol:.3e}"
+
+
+@pytest.mark.parametrize("W,D,B", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_products_in_columns(W, D, B, dtype):
+    # D + 2 terms of at most 1 in modulus: D + 3 roundings of partial sums of
+    # at most D + 2, and one of the result in the reference's rounding
+    tol = 2 * (D + 4) * (D + 2) * EPS[dtype]
+    rng = np.random.default_rng(100 * W + D)
+    st, basis = pkg.GB300Strategy(dtype), pkg.TensorBasis(W, D)
+    for pad, off in ((0, 0), (1, 1), (3, 2)):
+        for ro, rl, rr, ra in (((0, D), (0, D), (0, D), (0, D)), ((0, D - 1), (1, D), (0, D), (1, D - 1)),
+                               ((1, D), (0, D - 1), (1, 1), (0, 0)), ((D, D), (0, D), (D, D), (D, D))):
+            if min(ro[1], rl[1], rr[1], ra[1]) < 0 or ro[0] > ro[1]:
+                continue
+            out, a, b, c = (Rows(rng, dtype, W, D, B, pad, off) for _ in range(4))
+            ho, ha, hb, hc = (v.host() for v in (out, a, b, c))
+            prod = product(restrict(hb, W, D, rl), restrict(hc, W, D, rr), W, D)
+            assert pkg.ft_mul(st, None, out.view(*ro), b.view(*rl), c.view(*rr), basis, B)
+            check(out.host(), ho, prod, W, D, ro, tol)
+            before = out.host()
+            assert pkg.ft_fma(st, None, out.view(*ro), a.view(*ra), b.view(*rl), c.view(*rr), basis, B, 0.5, -0.75)
+            check(out.host(), before, 0.5 * restrict(ha, W, D, ra) - 0.75 * prod, W, D, ro, tol)
+            # in place: a = alpha c + beta a (x) b, b (x) a, and a = alpha a + beta b (x) c
+            for kind, rhs_first in ((1, False), (2, True), (0, None)):
+                x = Rows(rng, dtype, W, D, B, pad, off)
+                hx = x.host()
+                rx, ry = restrict(hx, W, D, ro), restrict(hb, W, D, rl)
+                if rhs_first is None:
+                    want = 0.5 * hx - 0.75 * prod
+                    third = c.view(*rr)
+                else:
+                    pr = product(ry, rx, W, D) if rhs_first else product(rx, ry, W, D)
+                    want = 0.5 * restrict(hc, W, D, ra) - 0.75 * pr
+                    third = c.view(*ra)
+                assert pkg.ft_inplace_fma(kind, st, None, x.view(*ro), b.view(*rl), third, basis, B, 0.5, -0.75)
+                check(x.host(), hx, want, W, D, ro, tol)
+            assert torch.all(out.buf[:off] == 7) and torch.all(out.buf[off:].view(B, -1)[:, out.n:] == 7)
