@@ -432,6 +432,9 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
                                 IntermediateKind kind, TArg<T> out, TArg<T> x, TArg<T> m,
                                 int64_t batch) {
     if (batch <= 0) return cudaSuccess;
+    if (kind != IntermediateKind::Log && chen_step_fits<T>(g, dev, out, x))
+        return launch_chen_step<T>(g, dev, s, out, kind == IntermediateKind::FMExp ? m : TArg<T>{nullptr, 0, 1, 0}, x,
+                                   batch, kind == IntermediateKind::Exp && out.lo == 0);
     constexpr auto kernel = k_intermediate<T>;
     cudaError_t err = allow_large_smem<kernel>(dev);
     if (err != cudaSuccess) return err;

@@ -34,12 +34,19 @@ cudaError_t launch_product(const Geometry& g, const DeviceInfo& dev, cudaStream_
                            double beta);
 
 // The column form of launch_product (widths 2..8, both factors in
-// shared memory) (ft_column.cu).
+// shared memory) and the one-pass form of exp / fmexp
+// for an exponent of degree one (ft_column.cu).
 template <typename T>
 bool column_product_fits(const Geometry& g, const DeviceInfo& dev);
 template <typename T>
 cudaError_t launch_column_product(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out, TArg<T> add,
                                 TArg<T> lhs, TArg<T> rhs, int64_t batch, double alpha, double beta);
+template <typename T>
+bool chen_step_fits(const Geometry& g, const DeviceInfo& dev, const TArg<T>& out, const TArg<T>& x);
+template <typename T>
+cudaError_t launch_chen_step(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out, TArg<T> mult,
+                             TArg<T> x, int64_t batch, bool unit);
+
 template <typename T>
 cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
                                 IntermediateKind kind, TArg<T> out, TArg<T> x, TArg<T> y,

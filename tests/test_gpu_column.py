@@ -1,5 +1,6 @@
 """The compile-time-width per-operation kernels against plain numpy in FP64:
-products a column of coefficients at a time (csrc/ft_column.cu), at the edges of their tasks --
+products a column of coefficients at a time (csrc/ft_column.cu) and the
+degree-one exponential step (csrc/ft_chen.cu), at the edges of their tasks --
 levels shorter than a column's first letters, partial last groups of tensors,
 strided and unaligned rows, degree ranges, every in-place form."""
 import importlib
@@ -99,3 +100,35 @@ def test_products_in_columns(W, D, B, dtype):
                 assert pkg.ft_inplace_fma(kind, st, None, x.view(*ro), b.view(*rl), third, basis, B, 0.5, -0.75)
                 check(x.host(), hx, want, W, D, ro, tol)
             assert torch.all(out.buf[:off] == 7) and torch.all(out.buf[off:].view(B, -1)[:, out.n:] == 7)
+
+
+@pytest.mark.parametrize("W,D,B", SHAPES + [(6, 6, 2)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_degree_one_exponential_step(W, D, B, dtype):
+    # M (x) exp(x) with |M| <= 1, |x_a| <= 1/2: every chain's partial values are
+    # below e, formed by at most D multiply-adds of D rounded letters each
+    tol = 3 * (2 * D + 4) * EPS[dtype]
+    rng = np.random.default_rng(10 * W + D)
+    st, basis, db = pkg.GB300Strategy(dtype), pkg.TensorBasis(W, D), starts(W, D)
+    xs = torch.from_numpy(rng.uniform(-0.5, 0.5, (B, W + 3))).to("cuda", dtype)
+    xb = pkg.make_tensor_batch(xs, W + 3, 1, 1, 1)  # letters in columns 2 .. W + 1
+    hx = np.zeros((B, db[-1]))
+    hx[:, 1:W + 1] = xs[:, 2:W + 2].double().cpu().numpy()
+    e = np.zeros_like(hx)
+    e[:, 0] = 1
+    power = e.copy()
+    for k in range(1, D + 1):
+        power = product(power, hx, W, D) / k
+        e += power
+    for pad, off in ((0, 0), (1, 1), (3, 2)):
+        for ro, rm in (((0, D), (0, D)), ((0, D), (1, D - 1)), ((1, D), (0, D)), ((0, D - 1), (0, D)), ((D, D), (0, D))):
+            if ro[1] < 1:
+                continue
+            out, m = (Rows(rng, dtype, W, D, B, pad, off) for _ in range(2))
+            ho = out.host()
+            want = product(restrict(restrict(m.host(), W, D, rm), W, D, ro), e, W, D)
+            assert pkg.ft_fmexp(st, None, out.view(*ro), m.view(*rm), xb, basis, B)
+            check(out.host(), ho, want, W, D, ro, tol)
+            before = out.host()
+            assert pkg.ft_exp(st, None, out.view(*ro), xb, basis, B)
+            check(out.host(), before, e if ro[0] == 0 else np.zeros_like(e), W, D, ro, tol)
