@@ -352,6 +352,14 @@ int rpp_gb_conversion_matrix(int32_t width, int32_t depth, int32_t which, int64_
  * S_{k-1} = S_k (x) exp(-dx_k) instead of storing them.  sig may be NULL
  * when only the gradient is wanted.
  *
+ * Equal-length batches too small to fill the GPU with one path per CTA are cut
+ * in time where that is faster (a rule on the shape, the batch and the length,
+ * whatever schedule is recorded for paths that run whole): pieces of the paths
+ * run at once and are joined by Chen's identity, through stream-ordered scratch
+ * of at most 256 MB (the paths run whole where it cannot be had).  The results
+ * are those of the whole path up to rounding, and the same for the same
+ * arguments.
+ *
  * rpp_gb_signature_backward: the reverse pass alone, from final signatures
  * `sig` (as produced by rpp_gb_signature) and cotangents `seed`.
  * ---------------------------------------------------------------------- */
@@ -388,8 +396,9 @@ int rpp_gb_signature_host(const rpp_gb_plan* plan, rpp_gb_stream stream, int32_t
  * runtimes that own all device memory through their own allocator and forbid
  * cudaMalloc / cudaMallocAsync from plugins, real-time loops that must not wait
  * on or grow a memory pool, and hosts that budget device memory up front.
- * Same arguments, results and numerics as rpp_gb_signature; the only scratch
- * it needs (the work counter and longest-first order of a ragged batch) lives
+ * Same arguments and numerics as rpp_gb_signature, and the same results (up to
+ * rounding where that entry cuts few long paths in time); the only scratch it
+ * needs (the work counter and longest-first order of a ragged batch) lives
  * in a fixed 8 MiB device array of the library, held by every GPU that loads
  * the library until the process exits.  Limits: a ragged batch of at most
  * 2,097,088 paths (RPP_GB_OUT_OF_BOUNDS beyond), and only shapes whose state

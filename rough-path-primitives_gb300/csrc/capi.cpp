@@ -322,16 +322,19 @@ int check_signature_args(const rpp_gb_plan* plan, const void* incr, const int64_
 template <typename T>
 int run_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const void* incr, const int64_t* offsets,
                   int64_t length, int64_t batch, void* sig, int64_t sig_stride, const void* seed,
-                  int64_t seed_stride, void* grad, bool forward, int threads = -1) {
+                  int64_t seed_stride, void* grad, bool forward, int threads = -1, int64_t whole_batch = 0) {
     if (int rc = check_signature_args<T>(plan, incr, offsets, length, sig, sig_stride, seed, seed_stride, grad,
                                          forward))
         return rc;
+    // an explicit schedule runs the paths whole; otherwise few long paths may
+    // be cut in time, whatever schedule is recorded for whole paths
+    if (threads >= 0) whole_batch = -1;
     if (threads < 0) threads = scheduled_threads(schedule_key(plan, dtype, forward, sig, seed, offsets));
     rpp_gb::PathBatch paths{offsets, length, batch};
     return cuda_status(rpp_gb::launch_signature<T>(plan->geometry, plan->device, s, static_cast<const T*>(incr),
                                                    paths, static_cast<T*>(sig), sig_stride,
                                                    static_cast<const T*>(seed), seed_stride, static_cast<T*>(grad),
-                                                   forward, threads),
+                                                   forward, threads, whole_batch),
                        "signature kernel");
 }
 
@@ -551,7 +554,8 @@ int run_signature_host(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, c
             rc = cuda_status(err, "host-to-device copy");
             break;
         }
-        rc = run_signature<T>(plan, st[i], dtype, d_incr, nullptr, length, nb, d_sig, dim, d_seed, dim, d_grad, true);
+        rc = run_signature<T>(plan, st[i], dtype, d_incr, nullptr, length, nb, d_sig, dim, d_seed, dim, d_grad, true, -1,
+                              batch);
         if (rc != RPP_GB_SUCCESS) break;
         if (sig)
             err = copy_rows(static_cast<char*>(sig) + b0 * sig_stride * ts, sig_stride * ts, d_sig, dim * ts, dim * ts,
@@ -823,6 +827,10 @@ int rpp_gb_plan_create(rpp_gb_plan** plan, int32_t width, int32_t depth, int32_t
     }
     p->geometry = g;
     p->device = info;
+    {
+        DeviceGuard guard(device);
+        rpp_gb::piece_scratch_retain(device);
+    }
     *plan = p;
     return ok();
 }
@@ -831,6 +839,7 @@ int rpp_gb_plan_destroy(rpp_gb_plan* plan) {
     if (plan && plan->geometry.fault) {
         DeviceGuard guard(plan->device.device);
         cudaFree(plan->geometry.fault);
+        rpp_gb::piece_scratch_release(plan->device.device);
     }
     delete plan;
     return ok();

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(256) k_intermediate(Geometry G, IntermediateKi
 // about 8 000 terms per output degree, most of them in the narrow degrees.
 template <typename T>
 __global__ void __launch_bounds__(256) k_adjoint(Geometry G, int left, TArg<T> out, TArg<T> op,
-                                                 TArg<T> arg, int64_t batch, int staged) {
+                                                 TArg<T> arg, int64_t batch, int64_t arg_group, int staged) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
     T* sm = reinterpret_cast<T*>(smem_raw + kBulkHeader);
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) k_adjoint(Geometry G, int left, TArg<T> o
     const uint32_t nt = blockDim.x, t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
         const T* P = op.at(b);
-        const T* A = arg.at(b);
+        const T* A = arg.at(arg_group == 1 ? b : b / arg_group);
         T* o = out.at(b);
         if (staged) {
             BulkStage<T> st(bar, phase);
@@ -451,7 +451,7 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
 
 template <typename T>
 cudaError_t launch_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool left,
-                           TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch) {
+                           TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch, int64_t arg_group) {
     if (batch <= 0) return cudaSuccess;
     constexpr auto kernel = k_adjoint<T>;
     cudaError_t err = allow_large_smem<kernel>(dev);
@@ -476,7 +476,7 @@ cudaError_t launch_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_
     const int threads = threads_for(g.pw[g.depth]);
     dim3 grid;
     if ((err = batch_grid(kernel, dev, threads, smem, batch, grid)) != cudaSuccess) return err;
-    kernel<<<grid, threads, smem, s>>>(g, left ? 1 : 0, out, op, arg, batch, staged);
+    kernel<<<grid, threads, smem, s>>>(g, left ? 1 : 0, out, op, arg, batch, arg_group, staged);
     return cudaGetLastError();
 }
 
@@ -531,7 +531,7 @@ cudaError_t launch_exp_letter_vjp(const Geometry& g, const DeviceInfo& dev, cuda
                                                 IntermediateKind, TArg<T>, TArg<T>, TArg<T>,       \
                                                 int64_t);                                          \
     template cudaError_t launch_adjoint<T>(const Geometry&, const DeviceInfo&, cudaStream_t, bool, \
-                                           TArg<T>, TArg<T>, TArg<T>, int64_t);                    \
+                                           TArg<T>, TArg<T>, TArg<T>, int64_t, int64_t);           \
     template cudaError_t launch_antipode<T>(const Geometry&, const DeviceInfo&, cudaStream_t,      \
                                             bool, TArg<T>, TArg<T>, int64_t);                      \
     template cudaError_t launch_helper<T>(const Geometry&, const DeviceInfo&, cudaStream_t,        \

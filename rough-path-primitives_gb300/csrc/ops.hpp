@@ -52,9 +52,10 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
                                 IntermediateKind kind, TArg<T> out, TArg<T> x, TArg<T> y,
                                 int64_t batch);
 
+// Entry b of the batch reads row b / arg_group of `arg`.
 template <typename T>
 cudaError_t launch_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool left,
-                           TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch);
+                           TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch, int64_t arg_group = 1);
 
 template <typename T>
 cudaError_t launch_antipode(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool sign,
@@ -203,10 +204,36 @@ constexpr int kScheduleMergedReverse = 1 << 27;
 // with kScheduleForwardTopGlobal the top level then lives in the signature
 // and seed rows.
 constexpr int kScheduleClusterShift = 28;
+// `whole_batch`: the paths of the caller's whole batch where `paths` is a part
+// of it (0: `paths` is all; -1: the paths run whole); the rule that cuts paths in
+// time depends on it, so that a batch computed in parts gives the bits of the
+// same batch computed at once.
 template <typename T>
 cudaError_t launch_signature(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
                              const T* incr, PathBatch paths, T* sig, int64_t sig_stride,
-                             const T* seed, int64_t seed_stride, T* grad, bool forward, int threads);
+                             const T* seed, int64_t seed_stride, T* grad, bool forward, int threads,
+                             int64_t whole_batch = 0);
+
+// Few long paths cut in time (signature_chunks.cu): the pieces per path of a
+// call (1: not cut), the pieces as a ragged
+// batch, and the rounds that join the pieces' signatures.  chunk_reduce: pieces' signatures s[path][c] (rows of `pitch`) are
+// multiplied together, the products overwriting them; the whole path's goes to
+// `sig`.  chunk_scan: p[path][c] = s_0 (x) .. (x) s_c and q[path][c] = s_{c+1}
+// (x) .. (x) s_{last} (the unit for the last), and p's last row to `sig` if given.
+template <typename T>
+int64_t signature_chunks(const Geometry& g, const DeviceInfo& dev, int64_t batch, int64_t length, bool reverse);
+// Scratch of the pieces (stream-ordered; freed with cudaFreeAsync) from a pool
+// that holds memory only while the device has plans: each plan retains it.
+void piece_scratch_retain(int device);
+void piece_scratch_release(int device);
+cudaError_t piece_scratch_alloc(int device, void** out, size_t bytes, cudaStream_t s);
+cudaError_t chunk_offsets(cudaStream_t s, int64_t* offsets, int64_t paths, int64_t length, int64_t chunks);
+template <typename T>
+cudaError_t chunk_reduce(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, T* pieces, int64_t pitch,
+                         int64_t paths, int64_t chunks, T* sig, int64_t sig_stride);
+template <typename T>
+cudaError_t chunk_scan(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const T* pieces, T* p, T* q,
+                       int64_t pitch, int64_t paths, int64_t chunks, T* sig, int64_t sig_stride);
 
 // kScheduleLetterWarps (bit 16 of an FP32 call's schedule without
 // kScheduleSplit, where bits 16-25 have no other use): the FP32 kernels with

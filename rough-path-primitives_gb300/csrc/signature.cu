@@ -329,6 +329,12 @@ SigLaunches plan_launches(bool forward, bool has_sig, bool has_seed, bool has_gr
     return l;
 }
 
+// Elements from one piece's tensor to the next (rows on 128-byte boundaries).
+template <typename T>
+int64_t piece_pitch(const Geometry& g) {
+    return (static_cast<int64_t>(g.dim) + 31) / 32 * 32;
+}
+
 // Runs the launches; a ragged batch's work counter is re-armed between them.
 template <typename T>
 cudaError_t run_launches(const SigGeometry& sg, const DeviceInfo& dev, cudaStream_t s, const T* incr,
@@ -346,13 +352,67 @@ cudaError_t run_launches(const SigGeometry& sg, const DeviceInfo& dev, cudaStrea
 
 }  // namespace
 
+// Few long paths, cut into `chunks` pieces in time (signature_chunks.cu): the
+// pieces' signatures, all at once; their products; and for the gradient the
+// reverse pass of every piece from its own end state (the product up to it) and
+// cotangent (the seed seen through the product after it).  Scratch: one tensor
+// per piece, three with a gradient.
+template <typename T>
+cudaError_t run_in_pieces(const SigGeometry& sg, const DeviceInfo& dev, cudaStream_t s, const T* incr,
+                          const PathBatch& paths, int64_t chunks, T* sig, int64_t sig_stride, const T* seed,
+                          int64_t seed_stride, T* grad, T* scratch) {
+    const Geometry& g = sg.g;
+    constexpr bool fp32 = std::is_same<T, float>::value;
+    const bool letters = fp32 && letter_warps_supported(g.width, g.depth);
+    const bool letters_rev = fp32 && letter_reverse_supported(g.width, g.depth);
+    const int64_t pitch = piece_pitch<T>(g), rows = paths.batch * chunks;
+    // the pieces as a ragged batch (the kernels take them as any other), their
+    // offsets after the tensors in the scratch
+    T* own = scratch;
+    int64_t* offsets = reinterpret_cast<int64_t*>(scratch + (grad ? 3 : 1) * rows * pitch);
+    const PathBatch pieces{offsets, 0, rows};
+    cudaError_t err = chunk_offsets(s, offsets, paths.batch, paths.length, chunks);
+    if (err == cudaSuccess) err = run_launches<T>(sg, dev, s, incr, pieces, own, pitch,
+                                                  static_cast<const T*>(nullptr), 0, static_cast<T*>(nullptr),
+                                                  plan_launches(true, true, false, false, 0, letters, letters_rev));
+    if (err != cudaSuccess) return err;
+    if (!grad) return chunk_reduce<T>(g, dev, s, own, pitch, paths.batch, chunks, sig, sig_stride);
+    T* before = own + rows * pitch;    // products up to and with each piece
+    T* after = before + rows * pitch;  // products of the pieces after each
+    if ((err = chunk_scan<T>(g, dev, s, own, before, after, pitch, paths.batch, chunks, sig, sig_stride)) != cudaSuccess)
+        return err;
+    T* cot = own;  // the pieces' own signatures are not needed any more
+    const int D = g.depth;
+    err = launch_adjoint<T>(g, dev, s, false, TArg<T>{cot, pitch, 0, D}, TArg<T>{after, pitch, 0, D},
+                            TArg<T>{const_cast<T*>(seed), seed_stride, 0, D}, rows, chunks);
+    if (err != cudaSuccess) return err;
+    return run_launches<T>(sg, dev, s, incr, pieces, before, pitch, cot, pitch, grad,
+                           plan_launches(false, true, true, true, 0, letters, letters_rev));
+}
+
 template <typename T>
 cudaError_t launch_signature(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const T* incr,
                              PathBatch paths, T* sig, int64_t sig_stride, const T* seed, int64_t seed_stride,
-                             T* grad, bool forward, int threads) {
+                             T* grad, bool forward, int threads, int64_t whole_batch) {
     if (paths.batch <= 0) return cudaSuccess;
     const SigGeometry sg = make_sig_geometry(g);
     constexpr bool fp32 = std::is_same<T, float>::value;
+    if (forward && whole_batch >= 0 && !paths.offsets) {
+        const int64_t chunks = signature_chunks<T>(g, dev, std::max(whole_batch, paths.batch), paths.length,
+                                                   grad != nullptr);
+        if (chunks > 1) {
+            T* scratch = nullptr;
+            const size_t bytes = static_cast<size_t>(grad ? 3 : 1) * paths.batch * chunks * piece_pitch<T>(g) * sizeof(T) +
+                                 (static_cast<size_t>(paths.batch) * chunks + 1) * sizeof(int64_t);
+            if (piece_scratch_alloc(dev.device, reinterpret_cast<void**>(&scratch), bytes, s) == cudaSuccess) {
+                cudaError_t err = run_in_pieces<T>(sg, dev, s, incr, paths, chunks, sig, sig_stride, seed, seed_stride,
+                                                   grad, scratch);
+                const cudaError_t ferr = cudaFreeAsync(scratch, s);
+                return err != cudaSuccess ? err : ferr;
+            }
+            cudaGetLastError();  // no memory for the pieces: the paths run whole
+        }
+    }
     const SigLaunches launches = plan_launches(forward, sig != nullptr, seed != nullptr, grad != nullptr, threads,
                                                fp32 && letter_warps_supported(g.width, g.depth),
                                                fp32 && letter_reverse_supported(g.width, g.depth));
@@ -481,9 +541,9 @@ template cudaError_t launch_signature_static_scratch<double>(const Geometry&, co
                                                              StaticScratchRefusal*);
 
 template cudaError_t launch_signature<float>(const Geometry&, const DeviceInfo&, cudaStream_t, const float*,
-                                             PathBatch, float*, int64_t, const float*, int64_t, float*, bool, int);
+                                             PathBatch, float*, int64_t, const float*, int64_t, float*, bool, int, int64_t);
 template cudaError_t launch_signature<double>(const Geometry&, const DeviceInfo&, cudaStream_t, const double*,
                                               PathBatch, double*, int64_t, const double*, int64_t, double*, bool,
-                                              int);
+                                              int, int64_t);
 
 }  // namespace rpp_gb
