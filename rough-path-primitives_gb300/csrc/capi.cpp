@@ -1409,13 +1409,15 @@ int rpp_gb_signature_group(rpp_gb_stream stream, const rpp_gb_signature_job* job
         // forward + reverse for depth >= 3), unless the caller asks for a
         // team size
         const bool letters = t == 0 && job.dtype == RPP_GB_F32 && 32 * g.width <= cta &&
-                             ((job.sig && !job.seed && rpp_gb::letter_warps_supported(g.width, g.depth)) ||
-                              (job.seed && rpp_gb::letter_reverse_supported(g.width, g.depth)));
+                             ((job.sig && !job.seed && rpp_gb::letter_group_supported(g.width, g.depth)) ||
+                              (job.seed && g.depth >= 3 && rpp_gb::letter_group_supported(g.width, g.depth)));
         if (letters) t = 32 * g.width;
         if (t == 0) {
             // the recorded schedule's (forward) CTA size and cotangent
             // workspace, else the heuristic
-            const int rec = scheduled_threads(schedule_key(job.plan, job.dtype, true, job.sig, job.seed, job.offsets));
+            int rec = scheduled_threads(schedule_key(job.plan, job.dtype, true, job.sig, job.seed, job.offsets));
+            if (job.dtype == RPP_GB_F32 && (rec & rpp_gb::kScheduleLetterWarps) && !(rec & rpp_gb::kScheduleSplit))
+                rec = 0;  // a warp-per-letter shape that has no team here
             t = rec & 1023;
             if (!(rec & rpp_gb::kScheduleSplit) && ((rec >> rpp_gb::kScheduleClusterShift) & 7) == 0)
                 cot = cot || (rec & rpp_gb::kScheduleCotangentGlobal) != 0;
@@ -1462,7 +1464,13 @@ int rpp_gb_signature_with_schedule(const rpp_gb_plan* plan, rpp_gb_stream stream
                                    int64_t sig_stride, const void* seed, int64_t seed_stride, void* grad,
                                    int32_t schedule) {
     if (schedule <= 0) return fail(RPP_GB_INVALID_ARGUMENT, "schedule must be positive");
-    return with_plan(plan, dtype, batch, [&] {
+    return with_plan(plan, dtype, batch, [&]() -> int {
+        // (the other shapes of the warp-per-letter kernels are taken by the
+        // default and by the autotuner only)
+        if (dtype == RPP_GB_F32 && (schedule & rpp_gb::kScheduleLetterWarps) && !(schedule & rpp_gb::kScheduleSplit) &&
+            rpp_gb::letter_warps_supported(plan->geometry.width, plan->geometry.depth) &&
+            !rpp_gb::letter_group_supported(plan->geometry.width, plan->geometry.depth))
+            return cuda_status(cudaErrorInvalidConfiguration, "signature kernel");
         auto s = static_cast<cudaStream_t>(stream);
         return dtype == RPP_GB_F64 ? run_signature<double>(plan, s, dtype, incr, offsets, length, batch, sig,
                                                            sig_stride, seed, seed_stride, grad, true, schedule)

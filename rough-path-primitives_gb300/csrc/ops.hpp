@@ -241,6 +241,10 @@ cudaError_t chunk_scan(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
 // (signature_fp32.cu) -- the forward-only kernel, and for calls with a
 // reverse pass (depth >= 3) the forward + reverse kernel.
 constexpr int kScheduleLetterWarps = 1 << 16;
+// Shapes with those kernels (letter_warps_supported: forward-only; also with a
+// reverse pass: letter_reverse_supported); letter_group_supported: the ones
+// that the grouped launch, and a schedule that asks for them, take.
+bool letter_group_supported(int width, int depth);
 bool letter_warps_supported(int width, int depth);
 bool letter_reverse_supported(int width, int depth);
 cudaError_t launch_signature_letters(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const float* incr,

@@ -373,7 +373,7 @@ __device__ __forceinline__ void letter_forward(const float* __restrict__ incr, i
                                                uint32_t lane, bool with_top) {
     using Lay = LetterLayout<W, D>;
     static_assert(D >= 2 && W <= 32, "one letter per lane");
-    static_assert(LetterLayout<W, D>::rows_per_lane * W <= 32, "at most 32 registers of top-level rows");
+    static_assert(LetterLayout<W, D>::rows_per_lane * W <= 48, "at most 48 registers of top-level rows");
     constexpr int R = Lay::rows_per_lane;
     for (uint32_t i = lane; i < Lay::s_size; i += 32) S[i] = 0.0f;
 #pragma unroll
@@ -935,12 +935,18 @@ __device__ __forceinline__ void letter_fwd_bwd(const Team& tm, const float* __re
     }
 }
 
-// The instantiated (width, depth) shapes, as X(width, depth) entries: at most
-// 32 registers of top-level rows per lane, and few enough lower-level
-// coefficients per lane to stay within 64 registers (W4 D6 and W3 D7 needed
-// 168 in an earlier form).
+// The instantiated (width, depth) shapes, as X(width, depth) entries: those
+// that the grouped launch instantiates too (at most 32 registers of top-level
+// rows per lane, and few enough lower-level coefficients per lane to stay
+// within 64 registers), and those that only single calls take (at most 48
+// registers of top rows; W4 D6 and W6 D5 run at 127 to 168 registers).  Deeper
+// tensors of widths 2 and 3 keep the shared-memory kernel: W2 D9, W2 D10 and
+// W3 D7 unroll into kernels that take minutes to compile.
 #define RPP_GB_LETTER_SHAPES(X) \
     X(8, 2) X(8, 3) X(8, 4) X(5, 2) X(5, 3) X(5, 4) X(5, 5) X(4, 4) X(4, 5) X(6, 4) X(3, 5) X(3, 6) X(16, 2)
+#define RPP_GB_LETTER_SHAPES_NARROW(X) \
+    X(2, 2) X(2, 3) X(2, 4) X(2, 5) X(2, 6) X(2, 7) X(3, 2) X(3, 3) X(3, 4)
+#define RPP_GB_LETTER_SHAPES_WIDE(X) X(4, 2) X(4, 3) X(4, 6) X(6, 2) X(6, 3) X(6, 5) X(7, 2) X(7, 3) X(7, 4)
 
 }  // namespace
 }  // namespace rpp_gb
