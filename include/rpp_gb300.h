@@ -352,6 +352,11 @@ int rpp_gb_conversion_matrix(int32_t width, int32_t depth, int32_t which, int64_
  * S_{k-1} = S_k (x) exp(-dx_k) instead of storing them.  sig may be NULL
  * when only the gradient is wanted.
  *
+ * A call without a recorded schedule takes one chosen from the shape, the batch
+ * and what it computes (CTA size, one launch or two, which arrays are kept in
+ * stream-ordered workspaces); outputs of different schedules agree up to
+ * rounding.
+ *
  * Equal-length batches too small to fill the GPU with one path per CTA are cut
  * in time where that is faster (a rule on the shape, the batch and the length,
  * whatever schedule is recorded for paths that run whole): pieces of the paths

@@ -829,7 +829,7 @@ int rpp_gb_plan_create(rpp_gb_plan** plan, int32_t width, int32_t depth, int32_t
     p->device = info;
     {
         DeviceGuard guard(device);
-        rpp_gb::piece_scratch_retain(device);
+        rpp_gb::scratch_retain(device);
     }
     *plan = p;
     return ok();
@@ -839,7 +839,7 @@ int rpp_gb_plan_destroy(rpp_gb_plan* plan) {
     if (plan && plan->geometry.fault) {
         DeviceGuard guard(plan->device.device);
         cudaFree(plan->geometry.fault);
-        rpp_gb::piece_scratch_release(plan->device.device);
+        rpp_gb::scratch_release(plan->device.device);
     }
     delete plan;
     return ok();

@@ -222,11 +222,11 @@ cudaError_t launch_signature(const Geometry& g, const DeviceInfo& dev, cudaStrea
 // (x) .. (x) s_{last} (the unit for the last), and p's last row to `sig` if given.
 template <typename T>
 int64_t signature_chunks(const Geometry& g, const DeviceInfo& dev, int64_t batch, int64_t length, bool reverse);
-// Scratch of the pieces (stream-ordered; freed with cudaFreeAsync) from a pool
-// that holds memory only while the device has plans: each plan retains it.
-void piece_scratch_retain(int device);
-void piece_scratch_release(int device);
-cudaError_t piece_scratch_alloc(int device, void** out, size_t bytes, cudaStream_t s);
+// Scratch of the signature calls (stream-ordered; freed with cudaFreeAsync) from
+// a pool that holds memory only while the device has plans: each plan retains it.
+void scratch_retain(int device);
+void scratch_release(int device);
+cudaError_t scratch_alloc(int device, void** out, size_t bytes, cudaStream_t s);
 cudaError_t chunk_offsets(cudaStream_t s, int64_t* offsets, int64_t paths, int64_t length, int64_t chunks);
 template <typename T>
 cudaError_t chunk_reduce(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, T* pieces, int64_t pitch,

@@ -193,7 +193,7 @@ cudaError_t launch_width(const SigGeometry& sg, const DeviceInfo& dev, cudaStrea
         if ((err = batch_grid(kernel, dev, threads, hsmem, paths.batch, grid)) != cudaSuccess) return err;
         const int64_t stride = static_cast<int64_t>((sg.g.db[sg.g.depth] + sg.chain_total + 31) / 32 * 32);
         T* ws = nullptr;
-        err = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(grid.x) * stride * sizeof(T), s);
+        err = scratch_alloc(dev.device, reinterpret_cast<void**>(&ws), static_cast<size_t>(grid.x) * stride * sizeof(T), s);
         if (err != cudaSuccess) return err;
         kernel<<<grid, threads, hsmem, s>>>(sg, incr, paths, sig, sig_stride, seed, seed_stride, grad, mode, ws, stride);
         err = cudaGetLastError();
@@ -248,7 +248,7 @@ cudaError_t launch_width(const SigGeometry& sg, const DeviceInfo& dev, cudaStrea
     smem = sig_smem_bytes<T>(sg, threads, bwd, false);
     const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(paths.batch, (two ? 2 : 1) * dev.sm_count));
     T* ws = nullptr;
-    cudaError_t err = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(ctas * stride) * sizeof(T), s);
+    cudaError_t err = scratch_alloc(dev.device, reinterpret_cast<void**>(&ws), static_cast<size_t>(ctas * stride) * sizeof(T), s);
     if (err != cudaSuccess) return err;
     kernel<<<dim3(static_cast<unsigned>(ctas)), threads, smem, s>>>(sg, incr, paths, sig, sig_stride, seed,
                                                                     seed_stride, grad, mode, ws, stride);
@@ -316,6 +316,8 @@ SigLaunches plan_launches(bool forward, bool has_sig, bool has_seed, bool has_gr
     } else {
         mode |= kBackward | kLoadFinal;
     }
+    // (a reverse pass alone: the seed's top level read from its row)
+    if (!forward && threads > 0 && (threads & kScheduleForwardTopGlobal)) mode |= kTopGlobal;
     // a forward-only call with kScheduleForwardTopGlobal keeps the top level
     // in the output row (the two-launch form's forward launch does the same)
     if (threads > 0 && (threads & kScheduleForwardTopGlobal) && mode == (kForward | kTopLevel) &&
@@ -327,6 +329,87 @@ SigLaunches plan_launches(bool forward, bool has_sig, bool has_seed, bool has_gr
                                                 (letters_rev && (mode & kBackward)));
     l.schedule[0] = letter_kernel ? (32 | kScheduleLetterWarps) : threads;
     return l;
+}
+
+// The schedule of a call without one (encoded as rpp_gb_signature_tune's; 0: the
+// heuristics of choose_variant, one launch).  What decides is how many paths an
+// SM runs at once.  A step is barrier-separated stages of a few coefficients a
+// thread, so an SM full of small CTAs, one path each, hides the stages that a
+// large CTA waits for: the fewest threads that still fill the SM, 1 024 over
+// the CTAs where shared memory limits them, 640 over the CTAs where the batch
+// does (many paths of a small state: one warp each).  Where the fused state of a
+// forward + reverse call keeps the SM from filling, the call runs as a forward
+// and a reverse launch, which hold less, the forward one with its top level in
+// the output row; and where the reverse launch alone still runs fewer than 8
+// CTAs per SM, its cotangent arrays go to the global workspace.  States of which
+// an SM holds one even so are split over a cluster.  FP64 reverse passes take
+// the D-barrier step.  Measured, 256-thread heuristics -> this rule, forward +
+// reverse, FP64 (ms): W4 D4 4 096 x 16 1.03 -> 0.35, W3 D5 1.40 -> 0.49, W5 D4
+// 1.23 -> 0.58, W5 D5 2.93 -> 2.50, W2 D10 4.81 -> 3.58, W2 D12 1 024 x 16 5.5 ->
+// 4.1, W6 D5 2.68 -> 1.39, W6 D6 500 x 16 6.8 -> 4.6; forward W4 D4 0.25 -> 0.085,
+// W5 D5 0.75 -> 0.65; 600 x 32 W4 D4 0.30 -> 0.23.  The top level stays on chip
+// where leaving it would not save a wave, in FP32 (W2 D12 900 x 16 forward 0.54
+// ms, 0.63 in the row) and for W = 7 and W > 8 (W7 D4 0.45, 0.49 in the row);
+// depths 1 and 2 keep the plain reverse step; FP32 with W a multiple of 4 keeps
+// the forms it has.
+template <typename T>
+int default_schedule(const SigGeometry& sg, const DeviceInfo& dev, int64_t batch, bool forward, bool has_sig,
+                     bool reverse) {
+    const Geometry& g = sg.g;
+    const int D = g.depth, W = g.width;
+    constexpr bool fp64 = std::is_same<T, double>::value;
+    if (D < 1 || (!fp64 && W % 4 == 0)) return 0;
+    const size_t dim = g.dim, lo = g.db[D], chains = sg.chain_total;
+    const int want = static_cast<int>(std::min<int64_t>(32, (batch + dev.sm_count - 1) / dev.sm_count));
+    auto bytes = [&](size_t state) { return (state + 2 * static_cast<size_t>((D + 1) * W) + 2 * D + 143) * sizeof(T); };
+    auto fit = [&](size_t state) -> int {  // CTAs per SM
+        const size_t b = bytes(state);
+        if (b + 64 + 384 * sizeof(T) > static_cast<size_t>(dev.max_smem_optin)) return 0;
+        return static_cast<int>(std::min<size_t>(32, (static_cast<size_t>(dev.max_smem_optin) + 1024) / (b + 1088)));
+    };
+    const int widest = threads_for(g.pw[D], 512);
+    const int least = (D * W + 31) / 32 * 32;
+    auto threads = [&](size_t state) {
+        const int n = fit(state);
+        int ideal = n <= want ? 1024 / n : 640 / want;
+        if ((W & (W - 1)) == 0 && ideal >= 128)  // (levels of W^n coefficients divide evenly)
+            ideal = ideal >= 512 ? 512 : ideal >= 256 ? 256 : 128;
+        const int most = std::min(widest, fp64 && bytes(state) > (size_t(64) << 10) ? 512 : 256);
+        return std::max(least, std::max(32, std::min(most, (ideal + 16) / 32 * 32)));
+    };
+    if (least > kResidentMaxThreads) return 0;
+    const bool rows = fp64 && (W <= 6 || W == 8) && W >= 2;  // a top level in the output row pays
+    const int cluster = W % 2 == 0 ? 2 : W % 3 == 0 ? 3 : 0;
+    const bool split_state = fit(lo + chains) < 2 && cluster > 0 && D >= 2 && fit((lo + chains) / cluster + 64) > 0;
+    const int in_cluster = 512 | kScheduleForwardTopGlobal | ((cluster - 1) << kScheduleClusterShift);
+    auto forward_part = [&]() -> int {
+        if (W >= 16) return std::max(least, threads_for(g.pw[D]));  // (W16 D3 900 x 16: 156 us, 175 with 128 threads)
+        const int full = fit(dim + chains), top = fit(lo + chains);
+        const auto waves = [&](int n) { return (want + n - 1) / n; };
+        if (full > 0 && (!rows || waves(full) <= waves(top))) return threads(dim + chains);
+        return top > 0 ? threads(lo + chains) | kScheduleForwardTopGlobal : 0;
+    };
+    if (!reverse) return split_state ? in_cluster : forward_part();
+    const int merged = fp64 && D >= 3 ? kScheduleMergedReverse : 0;
+    auto reverse_part = [&](int& flags) -> int {  // the reverse launch, the top levels in the rows
+        if (fit(2 * (lo + chains)) >= std::min(8, want)) {
+            flags = merged;
+            return threads(2 * (lo + chains));
+        }
+        flags = kScheduleCotangentGlobal;
+        return fit(lo + chains) > 0 ? threads(lo + chains) : 0;
+    };
+    int flags = 0;
+    if (!forward) {
+        const int t = reverse_part(flags);
+        return t > 0 ? t | flags | kScheduleForwardTopGlobal : 0;
+    }
+    const size_t fused = dim + lo + 2 * chains;
+    if (fit(fused) >= want || (!has_sig && fit(fused) >= 4)) return threads(fused) | merged;
+    if (!has_sig) return fit(dim + chains) > 0 ? threads(dim + chains) | kScheduleCotangentGlobal : 0;
+    if (split_state) return in_cluster | kScheduleCotangentGlobal;
+    const int f = forward_part(), r = reverse_part(flags);
+    return f > 0 && r > 0 ? kScheduleSplit | f | (r << kScheduleReverseShift) | flags : 0;
 }
 
 // Elements from one piece's tensor to the next (rows on 128-byte boundaries).
@@ -352,6 +435,38 @@ cudaError_t run_launches(const SigGeometry& sg, const DeviceInfo& dev, cudaStrea
 
 }  // namespace
 
+// The launches of a call under `threads`, or under the default schedule's where
+// that is 0 (chosen for `whole_batch` entries, of which these may be a part);
+// its workspace forms give way to the heuristics where they cannot run.
+template <typename T>
+cudaError_t run_call(const SigGeometry& sg, const DeviceInfo& dev, cudaStream_t s, const T* incr, PathBatch paths,
+                     T* sig, int64_t sig_stride, const T* seed, int64_t seed_stride, T* grad, bool forward,
+                     int threads, int64_t whole_batch) {
+    const Geometry& g = sg.g;
+    constexpr bool fp32 = std::is_same<T, float>::value;
+    const bool letters = fp32 && letter_warps_supported(g.width, g.depth);
+    const bool letters_rev = fp32 && letter_reverse_supported(g.width, g.depth);
+    const bool has_sig = sig != nullptr, reverse = seed != nullptr && grad != nullptr;
+    auto launches = [&](int t) {
+        return run_launches<T>(sg, dev, s, incr, paths, sig, sig_stride, seed, seed_stride, grad,
+                               plan_launches(forward, has_sig, seed != nullptr, grad != nullptr, t, letters,
+                                             letters_rev));
+    };
+    if (threads == 0 && !(reverse ? letters_rev : letters)) {
+        const int t = default_schedule<T>(sg, dev, whole_batch, forward, has_sig, reverse);
+        if (t > 0) {
+            const cudaError_t err = launches(t);
+            if (err != cudaErrorMemoryAllocation && err != cudaErrorInvalidConfiguration) return err;
+            cudaGetLastError();
+            if (paths.counter) {  // (taken by a launch that did run)
+                const cudaError_t zero = cudaMemsetAsync(paths.counter, 0, sizeof(unsigned int), s);
+                if (zero != cudaSuccess) return zero;
+            }
+        }
+    }
+    return launches(threads);
+}
+
 // Few long paths, cut into `chunks` pieces in time (signature_chunks.cu): the
 // pieces' signatures, all at once; their products; and for the gradient the
 // reverse pass of every piece from its own end state (the product up to it) and
@@ -359,12 +474,9 @@ cudaError_t run_launches(const SigGeometry& sg, const DeviceInfo& dev, cudaStrea
 // per piece, three with a gradient.
 template <typename T>
 cudaError_t run_in_pieces(const SigGeometry& sg, const DeviceInfo& dev, cudaStream_t s, const T* incr,
-                          const PathBatch& paths, int64_t chunks, T* sig, int64_t sig_stride, const T* seed,
-                          int64_t seed_stride, T* grad, T* scratch) {
+                          const PathBatch& paths, int64_t whole_batch, int64_t chunks, T* sig, int64_t sig_stride,
+                          const T* seed, int64_t seed_stride, T* grad, T* scratch) {
     const Geometry& g = sg.g;
-    constexpr bool fp32 = std::is_same<T, float>::value;
-    const bool letters = fp32 && letter_warps_supported(g.width, g.depth);
-    const bool letters_rev = fp32 && letter_reverse_supported(g.width, g.depth);
     const int64_t pitch = piece_pitch<T>(g), rows = paths.batch * chunks;
     // the pieces as a ragged batch (the kernels take them as any other), their
     // offsets after the tensors in the scratch
@@ -372,9 +484,9 @@ cudaError_t run_in_pieces(const SigGeometry& sg, const DeviceInfo& dev, cudaStre
     int64_t* offsets = reinterpret_cast<int64_t*>(scratch + (grad ? 3 : 1) * rows * pitch);
     const PathBatch pieces{offsets, 0, rows};
     cudaError_t err = chunk_offsets(s, offsets, paths.batch, paths.length, chunks);
-    if (err == cudaSuccess) err = run_launches<T>(sg, dev, s, incr, pieces, own, pitch,
-                                                  static_cast<const T*>(nullptr), 0, static_cast<T*>(nullptr),
-                                                  plan_launches(true, true, false, false, 0, letters, letters_rev));
+    if (err == cudaSuccess)
+        err = run_call<T>(sg, dev, s, incr, pieces, own, pitch, static_cast<const T*>(nullptr), 0,
+                          static_cast<T*>(nullptr), true, 0, whole_batch * chunks);
     if (err != cudaSuccess) return err;
     if (!grad) return chunk_reduce<T>(g, dev, s, own, pitch, paths.batch, chunks, sig, sig_stride);
     T* before = own + rows * pitch;    // products up to and with each piece
@@ -386,8 +498,8 @@ cudaError_t run_in_pieces(const SigGeometry& sg, const DeviceInfo& dev, cudaStre
     err = launch_adjoint<T>(g, dev, s, false, TArg<T>{cot, pitch, 0, D}, TArg<T>{after, pitch, 0, D},
                             TArg<T>{const_cast<T*>(seed), seed_stride, 0, D}, rows, chunks);
     if (err != cudaSuccess) return err;
-    return run_launches<T>(sg, dev, s, incr, pieces, before, pitch, cot, pitch, grad,
-                           plan_launches(false, true, true, true, 0, letters, letters_rev));
+    return run_call<T>(sg, dev, s, incr, pieces, before, pitch, cot, pitch, grad, false, 0,
+                       whole_batch * chunks);
 }
 
 template <typename T>
@@ -396,32 +508,28 @@ cudaError_t launch_signature(const Geometry& g, const DeviceInfo& dev, cudaStrea
                              T* grad, bool forward, int threads, int64_t whole_batch) {
     if (paths.batch <= 0) return cudaSuccess;
     const SigGeometry sg = make_sig_geometry(g);
-    constexpr bool fp32 = std::is_same<T, float>::value;
+    const int64_t whole = std::max(whole_batch, paths.batch);
     if (forward && whole_batch >= 0 && !paths.offsets) {
-        const int64_t chunks = signature_chunks<T>(g, dev, std::max(whole_batch, paths.batch), paths.length,
-                                                   grad != nullptr);
+        const int64_t chunks = signature_chunks<T>(g, dev, whole, paths.length, grad != nullptr);
         if (chunks > 1) {
             T* scratch = nullptr;
             const size_t bytes = static_cast<size_t>(grad ? 3 : 1) * paths.batch * chunks * piece_pitch<T>(g) * sizeof(T) +
                                  (static_cast<size_t>(paths.batch) * chunks + 1) * sizeof(int64_t);
-            if (piece_scratch_alloc(dev.device, reinterpret_cast<void**>(&scratch), bytes, s) == cudaSuccess) {
-                cudaError_t err = run_in_pieces<T>(sg, dev, s, incr, paths, chunks, sig, sig_stride, seed, seed_stride,
-                                                   grad, scratch);
+            if (scratch_alloc(dev.device, reinterpret_cast<void**>(&scratch), bytes, s) == cudaSuccess) {
+                cudaError_t err = run_in_pieces<T>(sg, dev, s, incr, paths, whole, chunks, sig, sig_stride, seed,
+                                                   seed_stride, grad, scratch);
                 const cudaError_t ferr = cudaFreeAsync(scratch, s);
                 return err != cudaSuccess ? err : ferr;
             }
             cudaGetLastError();  // no memory for the pieces: the paths run whole
         }
     }
-    const SigLaunches launches = plan_launches(forward, sig != nullptr, seed != nullptr, grad != nullptr, threads,
-                                               fp32 && letter_warps_supported(g.width, g.depth),
-                                               fp32 && letter_reverse_supported(g.width, g.depth));
     // Ragged batches: order the paths longest first and hand them out through
     // a work counter (stream-ordered scratch, released after the launch).
     void* scratch = nullptr;
     if (paths.offsets && paths.batch > 1) {
         const size_t bytes = 256 + static_cast<size_t>(paths.batch) * sizeof(int32_t);
-        cudaError_t err = cudaMallocAsync(&scratch, bytes, s);
+        cudaError_t err = scratch_alloc(dev.device, &scratch, bytes, s);
         if (err != cudaSuccess) return err;
         paths.counter = static_cast<unsigned int*>(scratch);
         paths.order = reinterpret_cast<int32_t*>(static_cast<char*>(scratch) + 256);
@@ -432,7 +540,8 @@ cudaError_t launch_signature(const Geometry& g, const DeviceInfo& dev, cudaStrea
             return err;
         }
     }
-    cudaError_t err = run_launches<T>(sg, dev, s, incr, paths, sig, sig_stride, seed, seed_stride, grad, launches);
+    cudaError_t err = run_call<T>(sg, dev, s, incr, paths, sig, sig_stride, seed, seed_stride, grad, forward, threads,
+                                  whole);
     if (scratch) {
         cudaError_t ferr = cudaFreeAsync(scratch, s);
         if (err == cudaSuccess) err = ferr;

@@ -156,13 +156,12 @@ int join_threads(const Geometry& g) {
     }
 }
 
-// The pieces' scratch comes from a memory pool of the library's own, one a
-// device, made with the device's first plan (so never inside a stream capture).
+// The scratch of the signature calls (pieces, ragged orders, workspaces) comes
+// from a memory pool of the library's own, one a device, made with the device's first plan (so never inside a stream capture).
 // The device's default pool gives its memory back at every synchronisation, and
-// mapping it again cost the next call 100 to 250 us; this one keeps what a call
-// may use (256 MB at most) while the device has a plan, and gives it back with
-// the last one.
-constexpr uint64_t kPieceScratch = uint64_t{256} << 20;
+// mapping it again cost the next call 100 to 250 us; this one keeps at most
+// 256 MB while the device has a plan, and gives it back with the last one.
+constexpr uint64_t kScratchKept = uint64_t{256} << 20;
 std::mutex g_pool_lock;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 int g_pool_users[kMaxDevices] = {};
@@ -173,7 +172,7 @@ void keep_at_most(cudaMemPool_t pool, uint64_t bytes) {
 
 }  // namespace
 
-void piece_scratch_retain(int device) {
+void scratch_retain(int device) {
     if (device < 0 || device >= kMaxDevices) return;
     std::lock_guard<std::mutex> guard(g_pool_lock);
     if (!g_pool[device]) {
@@ -186,10 +185,10 @@ void piece_scratch_retain(int device) {
             cudaGetLastError();
         }
     }
-    if (g_pool_users[device]++ == 0 && g_pool[device]) keep_at_most(g_pool[device], kPieceScratch);
+    if (g_pool_users[device]++ == 0 && g_pool[device]) keep_at_most(g_pool[device], kScratchKept);
 }
 
-void piece_scratch_release(int device) {
+void scratch_release(int device) {
     if (device < 0 || device >= kMaxDevices) return;
     std::lock_guard<std::mutex> guard(g_pool_lock);
     if (--g_pool_users[device] == 0 && g_pool[device]) {
@@ -198,7 +197,7 @@ void piece_scratch_release(int device) {
     }
 }
 
-cudaError_t piece_scratch_alloc(int device, void** out, size_t bytes, cudaStream_t s) {
+cudaError_t scratch_alloc(int device, void** out, size_t bytes, cudaStream_t s) {
     cudaMemPool_t pool = nullptr;
     if (device >= 0 && device < kMaxDevices) {
         std::lock_guard<std::mutex> guard(g_pool_lock);
@@ -216,7 +215,8 @@ cudaError_t piece_scratch_alloc(int device, void** out, size_t bytes, cudaStream
 // chains (one path, 1 000 increments, FP64: W3 D2 0.87 us, W3 D5 2.7, W5 D5
 // 4.0, W2 D10 6.4, W6 D5 5.8 forward, four times that with the reverse pass;
 // warp-per-letter 0.13 and 0.7 us); a call's joins cost 50 us and each round 5
-// at most (several launches of a call that is waited for).
+// at most (several launches of a call that is waited for), twice that with the
+// reverse pass.
 // Measured, forward + reverse, whole -> in pieces: FP64 W3 D5, 4 paths of 1 000,
 // 10.2 -> 0.24 ms; W5 D5 1 path of 1 000 16.3 -> 0.32, 100 paths 16.3 -> 5.8;
 // 64 increments, 8 paths 1.05 -> 0.23; W2 D10 FP32 1 path of 1 000 21.7 -> 0.29.
@@ -237,15 +237,15 @@ int64_t signature_chunks(const Geometry& g, const DeviceInfo& dev, int64_t batch
     const int64_t fit = static_cast<int64_t>(dev.max_smem_optin / std::max(1.0, state));
     const int64_t per_sm = letters ? 2 : std::max<int64_t>(1, std::min<int64_t>(4, fit));
     int64_t chunks = std::min(per_sm * dev.sm_count / batch, length / (letters ? 16 : 8));
-    // scratch: at most kPieceScratch
+    // scratch: at most kScratchKept
     const int64_t row = static_cast<int64_t>((reverse ? 3 : 1) * sizeof(T)) * (g.dim + 32);
-    chunks = std::min(chunks, static_cast<int64_t>(kPieceScratch) / row / batch);
+    chunks = std::min(chunks, static_cast<int64_t>(kScratchKept) / row / batch);
     if (chunks < 2) return 1;
     const int64_t piece = (length + chunks - 1) / chunks;
     chunks = (length + piece - 1) / piece;  // none empty
     int rounds = 0;
     while ((int64_t{1} << rounds) < chunks) ++rounds;
-    return step * static_cast<double>(length - piece) > 50.0 + 5.0 * rounds ? chunks : 1;
+    return step * static_cast<double>(length - piece) > (reverse ? 2.0 : 1.0) * (50.0 + 5.0 * rounds) ? chunks : 1;
 }
 
 cudaError_t chunk_offsets(cudaStream_t s, int64_t* offsets, int64_t paths, int64_t length, int64_t chunks) {

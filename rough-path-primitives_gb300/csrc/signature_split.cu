@@ -230,7 +230,7 @@ cudaError_t launch_split_kernel(const SigGeometry& sg, const LevelStarts& full, 
         // stream-ordered workspace released after the launch
         const int64_t stride = static_cast<int64_t>((sg.g.db[sg.g.depth] + sg.chain_total + 31) / 32 * 32);
         T* ws = nullptr;
-        err = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(n * P) * stride * sizeof(T), s);
+        err = scratch_alloc(dev.device, reinterpret_cast<void**>(&ws), static_cast<size_t>(n * P) * stride * sizeof(T), s);
         if (err != cudaSuccess) return err;
         err = cudaLaunchKernelEx(&cfg, kernel, sg, full, incr, paths, sig, sig_stride, seed, seed_stride, grad, mode,
                                  ws, stride);
