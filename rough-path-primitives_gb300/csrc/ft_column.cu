@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kColumnThreads) k_column_product(Geometry G, T
     T* sm = reinterpret_cast<T*>(smem_raw + kBulkHeader);
     const int D = G.depth, ohi = imin(out.hi, D);
     const uint32_t pd = staged_elems<T>(G.dim);
-    const uint32_t tasks = tensor_tasks<W>(G, out.lo, ohi);
+    const uint32_t tasks = tensor_tasks<T, W>(G, out.lo, ohi);
     const int lhi = imin(lhs.hi, D), rhi = imin(rhs.hi, D);
     uint32_t phase = 0;
     bulk_stage_init(bar);
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kColumnThreads) k_column_product(Geometry G, T
         for (uint32_t t = threadIdx.x; t < tasks * held; t += blockDim.x) {
             int n;
             uint32_t i, place;
-            locate_task<W>(G, t, held, ohi, n, i, place);
+            locate_task<T, W>(G, t, held, ohi, n, i, place);
             const T* l = staged_row(l0, sm, pd, lhs, b0, i, G);
             const T* r = staged_row(r0, sm + per * pd, pd, rhs, b0, i, G);
             T* o = out.at(b0 + i) + G.db[n];
@@ -129,7 +129,7 @@ cudaError_t launch_column_product(const Geometry& g, const DeviceInfo& dev, cuda
         int threads;
         const size_t slot = column_slot_bytes<T>(g);
         const size_t limit = std::min(kColumnSmemLimit, static_cast<size_t>(dev.max_smem_optin)) - kBulkHeader;
-        column_shape(tensor_tasks<W>(g, out.lo, out.hi), slot, limit, batch, dev.sm_count, per, threads);
+        column_shape(tensor_tasks<T, W>(g, out.lo, out.hi), slot, limit, batch, dev.sm_count, per, threads);
         const size_t smem = kBulkHeader + per * slot;
         const int64_t groups = (batch + per - 1) / per;
         const T al = static_cast<T>(alpha), be = static_cast<T>(beta);

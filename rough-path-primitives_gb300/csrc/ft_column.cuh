@@ -14,8 +14,10 @@
 // the same multiply-adds in the same order, so the results are the same bits.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
+#include "bulk_stage.cuh"
 #include "common.cuh"
 #include "ft_device.cuh"
 #include "launch_util.cuh"
@@ -31,10 +33,13 @@ constexpr uint32_t ipow(uint32_t w, int n) {
     return r;
 }
 
-// First letters of a column, and the coefficients they make (4 to 9).
-template <int W>
+// First letters of a column, and the coefficients they make.  FP32 (3 to 9) is
+// bound by loads and index arithmetic, which long columns save; FP64 by its
+// pipe, whose lanes short columns fill better (W3 D6: 81 columns of 9 on the
+// top level, or 243 of 3).
+template <typename T, int W>
 struct Column {
-    static constexpr int SC = W == 2 ? 3 : W == 3 ? 2 : 1;
+    static constexpr int SC = sizeof(T) == 8 ? (W == 2 ? 2 : 1) : (W == 2 ? 3 : W == 3 ? 2 : 1);
     static constexpr uint32_t NC = ipow(W, SC);
 };
 
@@ -43,28 +48,28 @@ constexpr bool column_width(int w) { return w >= 2 && w <= 8; }
 
 // Tasks of level n: a column per suffix of the levels of at least SC letters,
 // a single coefficient per word of the others.
-template <int W>
+template <typename T, int W>
 __host__ __device__ __forceinline__ uint32_t level_tasks(const Geometry& G, int n) {
-    return n >= Column<W>::SC ? G.pw[n - Column<W>::SC] : G.pw[n];
+    return n >= Column<T, W>::SC ? G.pw[n - Column<T, W>::SC] : G.pw[n];
 }
-template <int W>
+template <typename T, int W>
 __host__ __device__ __forceinline__ uint32_t tensor_tasks(const Geometry& G, int lo, int hi) {
     uint32_t t = 0;
-    for (int n = lo; n <= hi; ++n) t += level_tasks<W>(G, n);
+    for (int n = lo; n <= hi; ++n) t += level_tasks<T, W>(G, n);
     return t;
 }
 
 // Task i of the levels [lo, hi] of `per` tensors, top level first: the level,
 // the tensor and the task's place in its level.
-template <int W>
+template <typename T, int W>
 __device__ __forceinline__ void locate_task(const Geometry& G, uint32_t i, uint32_t per, int hi, int& n,
                                             uint32_t& tensor, uint32_t& place) {
     n = hi;
-    uint32_t tasks = level_tasks<W>(G, n);
+    uint32_t tasks = level_tasks<T, W>(G, n);
     while (i >= tasks * per) {
         i -= tasks * per;
         --n;
-        tasks = level_tasks<W>(G, n);
+        tasks = level_tasks<T, W>(G, n);
     }
     tensor = per == 1 ? 0u : i / tasks;
     place = per == 1 ? i : i % tasks;
@@ -74,9 +79,9 @@ __device__ __forceinline__ void locate_task(const Geometry& G, uint32_t i, uint3
 // c s of level n (n >= SC).
 template <typename T, int W>
 __device__ __forceinline__ void column_sum(const Geometry& G, const T* __restrict__ L, const T* __restrict__ R, int n,
-                                           uint32_t s, int kmin, int kmax, T (&acc)[Column<W>::NC]) {
-    constexpr int SC = Column<W>::SC;
-    constexpr uint32_t NC = Column<W>::NC;
+                                           uint32_t s, int kmin, int kmax, T (&acc)[Column<T, W>::NC]) {
+    constexpr int SC = Column<T, W>::SC;
+    constexpr uint32_t NC = Column<T, W>::NC;
     // splits inside the suffix: q = s / W^k, r = s % W^k
     uint32_t q = s, r = 0, p = 1;
     const int kend = imin(kmax, n - SC);
@@ -115,20 +120,126 @@ __device__ __forceinline__ void column_sum(const Geometry& G, const T* __restric
 template <typename T, int W, typename Store>
 __device__ __forceinline__ void task_product(const Geometry& G, const Opnd<T>& L, const Opnd<T>& R, int n,
                                              uint32_t place, Store&& store) {
-    constexpr uint32_t NC = Column<W>::NC;
-    if (n >= Column<W>::SC) {
+    constexpr uint32_t NC = Column<T, W>::NC;
+    if (n >= Column<T, W>::SC) {
         const int kmin = imax(imax(R.lo, 0), n - L.hi);
         const int kmax = imin(imin(R.hi, n), n - L.lo);
         T acc[NC];
 #pragma unroll
         for (uint32_t c = 0; c < NC; ++c) acc[c] = T(0);
         column_sum<T, W>(G, L.p, R.p, n, place, kmin, kmax, acc);
-        const uint32_t ws = G.pw[n - Column<W>::SC];
+        const uint32_t ws = G.pw[n - Column<T, W>::SC];
 #pragma unroll
         for (uint32_t c = 0; c < NC; ++c) store(c * ws + place, acc[c]);
     } else {
         store(place, ftdev::split_sum<false>(G, L, R, n, place));
     }
+}
+
+// exp or log of X (levels X.lo >= 1 .. X.hi, in shared memory) to degree H by
+// Horner's rule.  Round d = H .. 1 multiplies the running tensor by X; what the
+// later rounds read of it, and so what a round forms, are its levels up to
+// H - d + 1 only -- 22 k multiply-adds at W5 D5 in all, where rounds over whole
+// tensors take 57 k.  The running tensor alternates between two buffers of the
+// levels below H, one barrier a round; the last round's coefficients go to
+// store(n, index in the level, value), n = 1 .. H.  exp runs ft_device.cuh's
+// rescaled recursion (up to its depth limit) and divides by H! before the last
+// round, in what that round reads: the levels below H, not all of them.
+// Returns the result's level 0.  Ends with a barrier.
+template <typename T, int W, bool Log, typename Store>
+__device__ __forceinline__ T horner(const Geometry& G, int H, const Opnd<T>& X, T* cur, T* next, Store&& store) {
+    const auto& rc = ftdev::recip<T>();
+    const bool scaled = !Log && H <= ftdev::kScaledHornerMaxDepth;
+    T c = T(1);  // level 0 of the running tensor
+    if (Log) c = H > 0 ? (H % 2 == 0 ? -rc.inv[H] : rc.inv[H]) : T(0);
+    if (threadIdx.x == 0) cur[0] = c;
+    __syncthreads();
+    for (int d = H; d > 0; --d) {
+        const int t = H - d + 1;
+        const uint32_t tasks = tensor_tasks<T, W>(G, 1, t);
+        const Opnd<T> L{cur, 0, t - 1}, R{X.p, X.lo, imin(X.hi, t)};
+        if (Log) c = d > 1 ? ((d - 1) % 2 == 0 ? -rc.inv[d - 1] : rc.inv[d - 1]) : T(0);
+        else if (scaled) c *= rc.num[d];
+        for (uint32_t i = threadIdx.x; i < tasks; i += blockDim.x) {
+            int n;
+            uint32_t tensor, place;
+            locate_task<T, W>(G, i, 1, t, n, tensor, place);
+            task_product<T, W>(G, L, R, n, place, [&](uint32_t at, T v) {
+                if (d == 1) {
+                    store(n, at, v);
+                    return;
+                }
+                if constexpr (!Log) {
+                    // (wider tensors of that depth are not held in shared memory)
+                    if (W == 2 && !scaled) v *= rc.inv[d];
+                    if (scaled && d == 2) v *= rc.inv_fact[H];
+                }
+                next[G.db[n] + at] = v;
+            });
+        }
+        if (threadIdx.x == 0 && d > 1) next[0] = scaled && d == 2 ? c * rc.inv_fact[H] : c;
+        __syncthreads();
+        T* swap = cur;
+        cur = next;
+        next = swap;
+    }
+    return scaled ? c * rc.inv_fact[H] : c;  // (log: 0)
+}
+
+// The same with the whole result in X's buffer `x` (levels 0 .. H).
+// `buf`: both running buffers, `half` elements each.  Level H replaces X's,
+// which only its coefficients' own threads read; the levels below go to the
+// buffer that the last round does not read, and from there to x.  Ends with a
+// barrier.
+template <typename T, int W, bool Log>
+__device__ __forceinline__ void horner_in_place(const Geometry& G, int H, T* x, int xlo, int xhi, T* buf,
+                                                uint32_t half) {
+    // the last round reads the buffer of its parity and may fill the other
+    T* low = (H & 1) ? buf + half : buf;
+    const T unit = horner<T, W, Log>(G, H, Opnd<T>{x, xlo, xhi}, buf, buf + half, [&](int n, uint32_t at, T v) {
+        (n == H ? x : low)[G.db[n] + at] = v;
+    });
+    const uint32_t below = G.db[H];
+    for (uint32_t i = threadIdx.x; i < below; i += blockDim.x) x[i] = i == 0 ? unit : low[i];
+    if (H == 0 && threadIdx.x == 0) x[0] = unit;
+    __syncthreads();
+}
+
+// out = M (x) E on out's degrees, E at `e` to degree he, M staged at `m` (levels
+// mlo..mhi).
+template <typename T, int W>
+__device__ __forceinline__ void multiply_out(const Geometry& G, T* o, int olo, int ohi, const T* m, int mlo, int mhi,
+                                             const T* e, int he) {
+    const uint32_t tasks = tensor_tasks<T, W>(G, olo, ohi);
+    for (uint32_t t = threadIdx.x; t < tasks; t += blockDim.x) {
+        int n;
+        uint32_t i, place;
+        locate_task<T, W>(G, t, 1, ohi, n, i, place);
+        T* dst = o + G.db[n];
+        task_product<T, W>(G, Opnd<T>{m, mlo, mhi}, Opnd<T>{e, 0, he}, n, place,
+                           [&](uint32_t at, T v) { dst[at] = v; });
+    }
+}
+
+constexpr int kHornerThreads = 512;
+// CTAs of kHornerThreads whose registers fit an SM: the rounds' barriers want
+// many warps more than registers (42 a thread, W5 D5 FP64 log 189 us; 96 a
+// thread, 248 us), except where the columns then spill.
+template <typename T, int W>
+constexpr int kHornerBlocks = sizeof(T) == 8 && W >= 6 ? 2 : 3;
+constexpr size_t kHornerSmemLimit = 200 * 1024;
+
+// A thread per task of a tensor (one warp for the smallest, whose rounds then
+// wait for nobody), at most 256 while two CTAs fit an SM.
+template <typename T, int W>
+inline int horner_threads(const Geometry& g, size_t smem) {
+    const uint32_t tasks = (tensor_tasks<T, W>(g, 0, g.depth) + 31) / 32 * 32;
+    return static_cast<int>(std::min<uint32_t>(tasks, smem > 110 * 1024 ? kHornerThreads : 256u));
+}
+
+inline bool horner_fits(const Geometry& g, const DeviceInfo& dev, size_t smem) {
+    return column_width(g.width) && g.depth >= 1 &&
+           smem <= std::min(kHornerSmemLimit, static_cast<size_t>(dev.max_smem_optin));
 }
 
 // One launch over `groups` CTAs' worth of work, as many at once as fit.

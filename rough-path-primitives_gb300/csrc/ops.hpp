@@ -47,6 +47,13 @@ template <typename T>
 cudaError_t launch_chen_step(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out, TArg<T> mult,
                              TArg<T> x, int64_t batch, bool unit);
 
+// exp / log / fmexp on columns of coefficients (widths 2..8, ft_horner.cu).
+template <typename T>
+bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out);
+template <typename T>
+cudaError_t launch_column_horner(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, IntermediateKind kind,
+                                 TArg<T> out, TArg<T> x, TArg<T> m, int64_t batch);
+
 template <typename T>
 cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
                                 IntermediateKind kind, TArg<T> out, TArg<T> x, TArg<T> y,
@@ -161,6 +168,21 @@ template <typename T>
 cudaError_t launch_lie_exp(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const CsrDevice& m,
                            const T* lie, int64_t lie_stride, int lo, int hi, TArg<T> out, TArg<T> mult,
                            int64_t batch, double alpha);
+
+// The same on columns of coefficients (widths 2..8, lie_column.cu).
+template <typename T>
+bool column_log_to_lie_fits(const Geometry& g, const DeviceInfo& dev, int lo);
+template <typename T>
+cudaError_t launch_column_log_to_lie(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const CsrDevice& m,
+                                     TArg<T> x, int hi, T* out, int64_t out_stride, int64_t out_size, int64_t batch,
+                                     double alpha);
+template <typename T>
+bool column_lie_exp_fits(const Geometry& g, const DeviceInfo& dev, const CsrDevice& m, const TArg<T>& out,
+                         bool multiplier);
+template <typename T>
+cudaError_t launch_column_lie_exp(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const CsrDevice& m,
+                                  const T* lie, int64_t lie_stride, int lo, int hi, TArg<T> out, TArg<T> mult,
+                                  int64_t batch, double alpha);
 
 // Self-test of the bounded mbarrier wait (peak_probe.cu): one CTA waits,
 // with a short limit, for a transaction that nothing completes; the wait

@@ -41,11 +41,11 @@ __device__ void join(const Geometry& G, T* out, T* also, const T* L, const T* R,
         const T* r = st.add(sm + pd, R, 0, D, G);
         ok = st.commit(G.fault);
         if (!ok) return;
-        const uint32_t tasks = tensor_tasks<WT>(G, 0, D);
+        const uint32_t tasks = tensor_tasks<T, WT>(G, 0, D);
         for (uint32_t t = threadIdx.x; t < tasks; t += blockDim.x) {
             int n;
             uint32_t i, place;
-            locate_task<WT>(G, t, 1, D, n, i, place);
+            locate_task<T, WT>(G, t, 1, D, n, i, place);
             task_product<T, WT>(G, Opnd<T>{l, 0, D}, Opnd<T>{r, 0, D}, n, place, [&](uint32_t at, T v) {
                 out[G.db[n] + at] = v;
                 if (also) also[G.db[n] + at] = v;
@@ -146,10 +146,10 @@ cudaError_t with_join_width(const Geometry& g, const DeviceInfo& dev, F&& f) {
     return f(std::integral_constant<int, 0>{});
 }
 
-template <int W>
+template <typename T, int W>
 int join_threads(const Geometry& g) {
     if constexpr (W > 0) {
-        const uint32_t tasks = tensor_tasks<W>(g, 0, g.depth);
+        const uint32_t tasks = tensor_tasks<T, W>(g, 0, g.depth);
         return std::min(kJoinThreads, std::max(64, static_cast<int>((tasks + 31) / 32 * 32)));
     } else {
         return threads_for(g.pw[g.depth]);
@@ -264,7 +264,7 @@ cudaError_t chunk_reduce(const Geometry& g, const DeviceInfo& dev, cudaStream_t 
             // pieces c = 0, 2^{r+1}, ... with a partner c + 2^r
             const int64_t pairs = (chunks - (int64_t{1} << r) + (int64_t{2} << r) - 1) >> (r + 1);
             err = join_launch<&k_chunk_reduce<T, W>>(dev, s, dim3(static_cast<unsigned>(paths * pairs)),
-                                                     join_threads<W>(g), W > 0 ? join_smem<T>(g) : 0, g, pieces, pitch,
+                                                     join_threads<T, W>(g), W > 0 ? join_smem<T>(g) : 0, g, pieces, pitch,
                                                      chunks, pairs, r, sig, sig_stride);
         }
         return err;
@@ -279,7 +279,7 @@ cudaError_t chunk_scan(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
         cudaError_t err = cudaSuccess;
         for (int r = 0; (int64_t{1} << r) < chunks && err == cudaSuccess; ++r)
             err = join_launch<&k_chunk_scan<T, W>>(dev, s, dim3(static_cast<unsigned>(paths * chunks), 2),
-                                                   join_threads<W>(g), W > 0 ? join_smem<T>(g) : 0, g, pieces, p, q,
+                                                   join_threads<T, W>(g), W > 0 ? join_smem<T>(g) : 0, g, pieces, p, q,
                                                    pitch, chunks, r, sig, sig_stride);
         return err;
     });

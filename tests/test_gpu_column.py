@@ -132,3 +132,48 @@ def test_degree_one_exponential_step(W, D, B, dtype):
             before = out.host()
             assert pkg.ft_exp(st, None, out.view(*ro), xb, basis, B)
             check(out.host(), before, e if ro[0] == 0 else np.zeros_like(e), W, D, ro, tol)
+
+
+def power_series(x, W, D, coefficient):
+    """sum over k of coefficient(k) x^k, x without its degree 0."""
+    u = x.copy()
+    u[:, 0] = 0
+    total, power = np.zeros_like(x), np.zeros_like(x)
+    power[:, 0] = 1
+    for k in range(D + 1):
+        total += coefficient(k) * power
+        power = product(power, u, W, D)
+    return total
+
+
+@pytest.mark.parametrize("W,D,B", SHAPES + [(2, 13, 2)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_horner_in_columns(W, D, B, dtype):
+    # |x_w| <= 1/4: coefficients of exp and log sum the compositions of a word
+    # of n letters, at most 2^(n-1) products, each below 4^-parts: below 2 in
+    # sum; every round of D sums at most D + 1 terms
+    tol = 4 * (D + 1) * (D + 2) * EPS[dtype]
+    rng = np.random.default_rng(1000 * W + D)
+    st, basis = pkg.GB300Strategy(dtype), pkg.TensorBasis(W, D)
+    log_term = lambda k: 0.0 if k == 0 else (-1.0) ** (k + 1) / k  # noqa: E731
+    exp_term = lambda k: 1.0 / float(np.prod(np.arange(1, k + 1, dtype=np.float64)))  # noqa: E731
+    for pad, off in ((0, 0), (3, 1)):
+        x, m = Rows(rng, dtype, W, D, B, pad, off, 0.25), Rows(rng, dtype, W, D, B, pad, off)
+        for ro, rx, rm in (((0, D), (0, D), (0, D)), ((0, D - 1), (1, D), (1, D)), ((1, D), (2, D), (0, D - 1)),
+                           ((0, 0), (0, D), (0, 0)), ((D, D), (0, D), (1, D))):
+            if min(ro[1], rm[1]) < 0 or ro[0] > ro[1] or rx[0] > rx[1]:
+                continue
+            hx = restrict(x.host(), W, D, rx)
+            exp, log = power_series(hx, W, D, exp_term), power_series(hx, W, D, log_term)
+            zero = np.zeros_like(hx)
+            want = {"ft_exp": exp if ro[0] == 0 else zero, "ft_log": log if ro[0] == 0 else zero}
+            for name, value in want.items():
+                out = Rows(rng, dtype, W, D, B, pad, off)
+                before = out.host()
+                assert getattr(pkg, name)(st, None, out.view(*ro), x.view(*rx), basis, B)
+                check(out.host(), before, value, W, D, ro, tol)
+            out = Rows(rng, dtype, W, D, B, pad, off)
+            before = out.host()
+            held = restrict(restrict(m.host(), W, D, rm), W, D, ro)
+            assert pkg.ft_fmexp(st, None, out.view(*ro), m.view(*rm), x.view(*rx), basis, B)
+            check(out.host(), before, product(held, exp, W, D), W, D, ro, tol * (D + 1))
