@@ -59,6 +59,13 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
                                 IntermediateKind kind, TArg<T> out, TArg<T> x, TArg<T> y,
                                 int64_t batch);
 
+// The adjoint multiplies for widths 2..8 (ft_adjoint.cu; `staged` as launch_adjoint
+// chooses it).
+bool column_adjoint_width(int width);
+template <typename T>
+cudaError_t launch_column_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool left, TArg<T> out,
+                                  TArg<T> op, TArg<T> arg, int64_t batch, int64_t arg_group, int staged);
+
 // Entry b of the batch reads row b / arg_group of `arg`.
 template <typename T>
 cudaError_t launch_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool left,

@@ -177,3 +177,41 @@ def test_horner_in_columns(W, D, B, dtype):
             held = restrict(restrict(m.host(), W, D, rm), W, D, ro)
             assert pkg.ft_fmexp(st, None, out.view(*ro), m.view(*rm), x.view(*rx), basis, B)
             check(out.host(), before, product(held, exp, W, D), W, D, ro, tol * (D + 1))
+
+
+def adjoint(p, a, W, D, left):
+    """out[m] = sum over p of the op's degree p against the argument's degree m + p."""
+    db, out = starts(W, D), np.zeros_like(a)
+    for m in range(D + 1):
+        for k in range(D - m + 1):
+            op, arg = p[:, db[k]:db[k + 1]], a[:, db[m + k]:db[m + k + 1]]
+            if left:
+                part = (op[:, None, :] @ arg.reshape(len(a), W ** k, W ** m))[:, 0]
+            else:
+                part = (arg.reshape(len(a), W ** m, W ** k) @ op[:, :, None])[:, :, 0]
+            out[:, db[m]:db[m + 1]] += part
+    return out
+
+
+@pytest.mark.parametrize("W,D,B", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_adjoints_in_columns(W, D, B, dtype):
+    rng = np.random.default_rng(7 * W + D)
+    st, basis = pkg.GB300Strategy(dtype), pkg.TensorBasis(W, D)
+    n = int(starts(W, D)[-1])
+    # sums of up to n terms of modulus at most 1, in any order: n roundings of
+    # partial sums that grow as the square root of their number (times 4), or
+    # linearly at worst for the few terms of small tensors
+    tol = 4 * np.sqrt(n) * min(n, 4 * np.sqrt(n) + 16) * EPS[dtype]
+    for pad, off in ((0, 0), (3, 1)):
+        op, arg = (Rows(rng, dtype, W, D, B, pad, off) for _ in range(2))
+        for ro, rp, ra in (((0, D), (0, D), (0, D)), ((0, D - 1), (1, D), (1, D - 1)), ((1, D), (0, 1), (0, D)),
+                           ((0, D), (D, D), (1, D)), ((D, D), (0, 0), (0, D))):
+            if min(ro[1], rp[1], ra[1]) < 0 or ro[0] > ro[1] or ra[0] > ra[1]:
+                continue
+            hp, ha = restrict(op.host(), W, D, rp), restrict(arg.host(), W, D, ra)
+            for name, left in (("ft_adj_lmul", True), ("ft_adj_rmul", False)):
+                out = Rows(rng, dtype, W, D, B, pad, off)
+                before = out.host()
+                assert getattr(pkg, name)(st, None, out.view(*ro), op.view(*rp), arg.view(*ra), basis, B)
+                check(out.host(), before, adjoint(hp, ha, W, D, left), W, D, ro, tol)
