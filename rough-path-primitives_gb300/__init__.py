@@ -86,10 +86,26 @@ def _status(rc: int) -> Error:
     return Error(ErrorCode(rc), msg.decode() if msg else "")
 
 
-def _torch():
-    import torch
+_torch_module = None
 
-    return torch
+
+def _torch():
+    global _torch_module
+    if _torch_module is None:
+        import torch
+
+        _torch_module = torch
+    return _torch_module
+
+
+def _raw_stream():
+    """device -> raw handle of torch's current stream, by the shortest way this torch has."""
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw if raw is not None else lambda device: torch.cuda.current_stream(device).cuda_stream
+
+
+_current_raw_stream = None
 
 
 _F32, _F64 = 0, 1
@@ -227,7 +243,7 @@ class GB300Strategy:
     device: int = 0
 
     def dtype_code(self) -> int:
-        torch = _torch()
+        torch = _torch_module or _torch()
         acc = self.accum if self.accum is not None else torch.float64
         if acc == torch.float64:
             return _F64
@@ -236,8 +252,7 @@ class GB300Strategy:
         raise ValueError("GB300Strategy supports float32 and float64")
 
     def torch_dtype(self):
-        torch = _torch()
-        return self.accum if self.accum is not None else torch.float64
+        return self.accum if self.accum is not None else _torch().float64
 
 
 @dataclass
@@ -252,8 +267,12 @@ class DeviceLaunchConfig:
     def handle(self, device: int) -> int:
         s = self.stream
         if s is None:
-            torch = _torch()
-            return torch.cuda.current_stream(device).cuda_stream
+            global _current_raw_stream
+            if _current_raw_stream is None:
+                torch = _torch()
+                torch.cuda.current_stream(device)  # CUDA is initialised from here on
+                _current_raw_stream = _raw_stream()
+            return _current_raw_stream(device)
         if isinstance(s, int):
             return s
         return s.cuda_stream
@@ -268,11 +287,14 @@ class FTInplaceFMAType(enum.IntEnum):
 
 
 def _check_batches(strategy: GB300Strategy, *batches):
+    _torch()
     dt = strategy.torch_dtype()
     for b in batches:
         if b is None:
             continue
         t = b.data
+        if t.__class__ is _torch_module.Tensor and t.is_cuda and t.dtype is dt:
+            continue
         if not getattr(t, "is_cuda", False):
             raise ValueError("batch data must be a CUDA tensor (the GB300 strategy has no host path)")
         if t.dtype != dt:
@@ -283,8 +305,11 @@ def _p(b):
     return None if b is None else ctypes.byref(b.arg())
 
 
+_default_config = DeviceLaunchConfig()
+
+
 def _cfg(config):
-    return config if config is not None else DeviceLaunchConfig()
+    return config if config is not None else _default_config
 
 
 # --------------------------------------------------------------------------

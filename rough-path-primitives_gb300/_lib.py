@@ -125,6 +125,8 @@ def build(jobs: int = 8) -> None:
 def load(path: str = LIB_PATH):
     """Load the shared library once; raise if it has not been built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(path):

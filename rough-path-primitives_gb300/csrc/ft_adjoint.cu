@@ -51,7 +51,7 @@ AdjointTasks adjoint_tasks(const Geometry& g, bool left, bool fp64, int olo, int
         const int top = std::min(phi, ahi - m), low = std::max(plo, alo - m);
         const uint32_t terms = low > top ? 1u : g.db[top + 1] - g.db[low];
         // (a warp's sum takes five additions more, dear in FP64)
-        if (wm < 32u && (left ? terms * wm : terms) >= (fp64 && !left && wm >= 8u ? 256u : 64u)) {
+        if (wm < 32u && (left ? terms * wm : terms) >= (!left && wm >= 8u ? 256u : 64u)) {
             at += left ? 1u : wm;
             continue;
         }

@@ -30,13 +30,37 @@ inline cudaError_t allow_large_smem(const DeviceInfo& dev) {
     return err;
 }
 
+// CTAs of a launch shape that fit an SM.  The runtime's query takes about as
+// long as a small launch, so each host thread remembers its answers (they depend
+// on the kernel, the device and the shape alone) in a small direct-mapped table.
+template <typename Kernel>
+inline cudaError_t ctas_per_sm(Kernel kernel, const DeviceInfo& dev, int threads, size_t smem, int& per_sm) {
+    struct Answer {
+        const void* kernel;
+        size_t smem;
+        int device, threads, per_sm;
+    };
+    static thread_local Answer answers[16] = {};  // (one table per kernel signature)
+    const void* key = reinterpret_cast<const void*>(kernel);
+    const size_t mixed = (reinterpret_cast<uintptr_t>(key) >> 4) + (smem >> 4) + static_cast<size_t>(threads >> 5);
+    Answer& a = answers[mixed % 16];
+    if (a.kernel != key || a.smem != smem || a.device != dev.device || a.threads != threads) {
+        int n = 0;
+        const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+        if (err != cudaSuccess) return err;
+        a = Answer{key, smem, dev.device, threads, n};
+    }
+    per_sm = a.per_sm;
+    return cudaSuccess;
+}
+
 // Grid for a "one CTA per batch element, grid-stride over the batch" kernel:
 // as many CTAs as fit on the device at once, capped by the batch.
 template <typename Kernel>
 inline cudaError_t batch_grid(Kernel kernel, const DeviceInfo& dev, int threads, size_t smem,
                               int64_t batch, dim3& grid) {
     int per_sm = 0;
-    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+    cudaError_t err = ctas_per_sm(kernel, dev, threads, smem, per_sm);
     if (err != cudaSuccess) return err;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int64_t cap = static_cast<int64_t>(per_sm) * dev.sm_count;
