@@ -125,8 +125,12 @@ cudaError_t launch_chen_step(const Geometry& g, const DeviceInfo& dev, cudaStrea
         constexpr int W = decltype(w)::value;
         const bool staged = mult.p != nullptr && chen_smem<T>(g, out.hi, true) <= kChenStageLimit;
         const size_t smem = chen_smem<T>(g, out.hi, staged);
-        // four coefficients of the widest level a thread; larger CTAs where few fit an SM
-        const int threads = std::max(64, threads_for(g.pw[out.hi] / 4, smem > 64 * 1024 ? 512 : 256));
+        // 14 (FP64) or 28 coefficients of the widest level a thread: what bounds small
+        // tensors is the stages' latency, which more and smaller CTAs an SM hide
+        // (W3 D6 batch 3000 FP32: 256 threads 17 us, 128 threads 12, 32 threads 9)
+        const uint32_t each = sizeof(T) == 8 ? 14 : 28;
+        const int threads = std::max(32, std::min(smem > 64 * 1024 ? 512 : 256,
+                                                  static_cast<int>((g.pw[out.hi] / each + 31) / 32 * 32)));
         return run_column<&k_chen_step<T, W>>(dev, s, threads, smem, batch, g, out, mult, x, batch, unit ? 1 : 0,
                                               staged ? 1 : 0);
     });
