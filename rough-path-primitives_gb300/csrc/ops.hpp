@@ -154,6 +154,22 @@ template <typename T>
 cudaError_t launch_shuffle_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ShuffleAdjKind kind,
                                    TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch, double beta);
 
+// The shuffle product and its adjoint a letter at a time (widths 2..8,
+// shuffle_letters.cu).
+template <typename T>
+bool shuffle_letters_product_fits(const Geometry& g, const DeviceInfo& dev, ShuffleKind kind, const TArg<T>& out,
+                                  const TArg<T>& add, const TArg<T>& lhs, const TArg<T>& rhs, int64_t batch);
+template <typename T>
+cudaError_t launch_shuffle_letters_product(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ShuffleKind kind,
+                                           TArg<T> out, TArg<T> add, TArg<T> lhs, TArg<T> rhs, int64_t batch,
+                                           double alpha, double beta);
+template <typename T>
+bool shuffle_letters_adjoint_fits(const Geometry& g, const DeviceInfo& dev, ShuffleAdjKind kind, const TArg<T>& out,
+                                  const TArg<T>& op, const TArg<T>& arg, int64_t batch);
+template <typename T>
+cudaError_t launch_shuffle_letters_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out,
+                                           TArg<T> op, TArg<T> arg, int64_t batch);
+
 template <typename T>
 cudaError_t launch_pairing(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, T* result, TArg<T> f, TArg<T> a,
                            int64_t batch);

@@ -718,6 +718,8 @@ cudaError_t launch_shuffle_product(const Geometry& g, const DeviceInfo& dev, cud
                                    TArg<T> out, TArg<T> add, TArg<T> lhs, TArg<T> rhs, int64_t batch, double alpha,
                                    double beta, const ShuffleOrder& ord) {
     if (batch <= 0 || ord.start[ord.count] == 0) return cudaSuccess;
+    if (shuffle_letters_product_fits<T>(g, dev, kind, out, add, lhs, rhs, batch))
+        return launch_shuffle_letters_product<T>(g, dev, s, kind, out, add, lhs, rhs, batch, alpha, beta);
     if (g.depth > 30) return cudaErrorInvalidValue;
     int threads, staged;
     size_t smem;
@@ -749,6 +751,8 @@ template <typename T>
 cudaError_t launch_shuffle_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ShuffleAdjKind kind,
                                    TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch, double beta) {
     if (batch <= 0) return cudaSuccess;
+    if (shuffle_letters_adjoint_fits<T>(g, dev, kind, out, op, arg, batch) && static_cast<T>(beta) == T(1))
+        return launch_shuffle_letters_adjoint<T>(g, dev, s, out, op, arg, batch);
     auto run = [&](auto kernel_c) -> cudaError_t {
         constexpr auto kernel = decltype(kernel_c)::value;
         cudaError_t err = allow_large_smem<kernel>(dev);
