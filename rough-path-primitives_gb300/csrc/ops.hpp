@@ -154,7 +154,7 @@ template <typename T>
 cudaError_t launch_shuffle_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ShuffleAdjKind kind,
                                    TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch, double beta);
 
-// The shuffle product and its adjoint a letter at a time (widths 2..8,
+// The shuffle and half-shuffle products and their adjoints a letter at a time (widths 2..8,
 // shuffle_letters.cu).
 template <typename T>
 bool shuffle_letters_product_fits(const Geometry& g, const DeviceInfo& dev, ShuffleKind kind, const TArg<T>& out,
@@ -167,8 +167,9 @@ template <typename T>
 bool shuffle_letters_adjoint_fits(const Geometry& g, const DeviceInfo& dev, ShuffleAdjKind kind, const TArg<T>& out,
                                   const TArg<T>& op, const TArg<T>& arg, int64_t batch);
 template <typename T>
-cudaError_t launch_shuffle_letters_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out,
-                                           TArg<T> op, TArg<T> arg, int64_t batch);
+cudaError_t launch_shuffle_letters_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
+                                           ShuffleAdjKind kind, TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch,
+                                           double beta);
 
 template <typename T>
 cudaError_t launch_pairing(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, T* result, TArg<T> f, TArg<T> a,

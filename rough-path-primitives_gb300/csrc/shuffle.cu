@@ -751,8 +751,8 @@ template <typename T>
 cudaError_t launch_shuffle_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ShuffleAdjKind kind,
                                    TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch, double beta) {
     if (batch <= 0) return cudaSuccess;
-    if (shuffle_letters_adjoint_fits<T>(g, dev, kind, out, op, arg, batch) && static_cast<T>(beta) == T(1))
-        return launch_shuffle_letters_adjoint<T>(g, dev, s, out, op, arg, batch);
+    if (shuffle_letters_adjoint_fits<T>(g, dev, kind, out, op, arg, batch))
+        return launch_shuffle_letters_adjoint<T>(g, dev, s, kind, out, op, arg, batch, beta);
     auto run = [&](auto kernel_c) -> cudaError_t {
         constexpr auto kernel = decltype(kernel_c)::value;
         cudaError_t err = allow_large_smem<kernel>(dev);

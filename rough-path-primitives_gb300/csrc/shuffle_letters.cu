@@ -1,26 +1,30 @@
-// shuffle_letters.cu -- the shuffle product (st_mul, st_fma, st_inplace_fma) and
-// its adjoint (st_adj_mul) a letter at a time, for widths 2..8.
+// shuffle_letters.cu -- the shuffle algebra a letter at a time, for widths 2..8:
+// st_mul, st_fma, st_inplace_fma, left_hs_mul and their adjoints.
 //
 // The subset sums of shuffle.cu take 2^N terms for a word of N letters.  Dealing
 // the letters of a word one by one to the two factors instead shares all but
-// N^2 / 2 of them.  Adjoint: with
-//     E_m^k[u, v, r] = sum over interleavings s of u and v of arg[s r],
-// |u| = k, |v| = m - k, r the N - m letters not yet dealt,
-//     E_{m+1}^k[u, v, r] = E_m^{k-1}[u', v, a r] + E_m^k[u, v', b r],
-// u = u' a, v = v' b, and out[v] = sum_u op[u] E_N^k[u, v].  Stored as one array of
-// W^N per k in the order u v r, the second term is the same place of the array
-// (v takes in the letter beside it), so a step adds E^{k-1}, with the letter a
-// moved past v, into E^k; E^0 and E^m are the argument itself.  At N = 5 that is
-// 10 additions and 6 multiply-adds a word where the subsets take 32
-// multiply-adds, at N = 8 28 and 9 against 256.
-// The product is the transpose: E^k starts as L_k (x) R_{N-k} and every step adds
-// E^k, the letter moved back, into E^{k-1}.
-// A CTA owns a tensor and keeps the N arrays of one degree in shared memory, a
-// barrier between the steps, which with the index instructions is what bounds it.
-// Product / adjoint, by subsets -> by letters (us): FP64 W2 D8 batch 4096 652 ->
-// 211 / 2570 -> 249, W3 D6 batch 3000 312 -> 203 / 661 -> 279, W4 D4 batch 1024
-// 16.5 -> 15.7 / 43 -> 22; FP32 W2 D8 338 -> 118 / 2342 -> 156, W3 D6 172 -> 119 /
-// 604 -> 181, W5 D5 batch 4096 496 -> 406 / 686 -> 644.
+// N^2 / 2 of them.  Adjoint: for a word c s of degree N = M + 1 and arrays over s,
+//     E_m^k[r, v, u] = sum over interleavings t of u and v of arg[c r t],
+// |u| = k, |v| = m - k, r the M - m letters not yet dealt (last letters first),
+//     E_{m+1}^k[r, v, u] = E_m^k[r b, v', u] + E_m^{k-1}[r a, v, u'],
+// v = b v', u = a u', and the first letter is dealt last,
+//     out[v] += op[c u] E_M^k[v, u],   out[c v] += op[u] E_M^k[v, u],
+// summed over u and c (the half-shuffle adjoints take one of the two).  Stored as
+// one array of W^M per k in the order r v u, the first term of a step is the same
+// place of the array (v takes in the letter beside it), so a step adds E^{k-1},
+// with the letter a moved past v, into E^k; E^0 and E^m are the argument itself.
+// At N = 5 that is 16 operations a word where the subsets take 32, at N = 8 37
+// against 256.  The product is the transpose: E_M^k = L[c u] R[v] + L[u] R[c v]
+// (the half-shuffle product: the first), and every step adds E^k, the letter
+// moved back, into E^{k-1}.
+// A CTA owns a tensor and keeps the arrays of one degree and one first letter (all
+// first letters, where they fit) in shared memory, a barrier between the steps;
+// these and the index instructions are what bounds it.  Subsets -> letters (us),
+// batch 4096 unless said: st_mul FP64 W5 D5 832 -> 687, W6 D5 (2048) 1432 -> 911, W2
+// D8 652 -> 181, FP32 W5 D5 496 -> 333, W8 D4 376 -> 262; st_adj_mul FP64 W2 D8 2570 ->
+// 418, W3 D6 (3000) 661 -> 376, FP32 W5 D5 686 -> 479, W2 D8 2342 -> 161; left_hs_mul
+// FP32 W4 D3 (8192) 17.7 -> 8.9; left_hs_adj_lmul / _rmul W2 D8 FP64 1032 -> 264 / 1771
+// -> 302, FP32 935 -> 144 / 1633 -> 150.
 #include <algorithm>
 #include <type_traits>
 
@@ -59,171 +63,234 @@ __device__ __forceinline__ uint32_t letter_back(const Geometry& G, const PowerDi
     return ((up * W + a) * G.pw[b] + v) * G.pw[R] + r;
 }
 
-// Coefficients of the degrees that a warp or less of lanes covers: their sums
-// over u are shared by all warps and added up in warp order.
-template <int W>
-constexpr uint32_t kNarrow = W == 2 ? 31u : W == 3 ? 40u : W == 4 ? 21u : W == 5 ? 31u : W + 1u;
+// The letter step's arrays of `block` first letters (the argument or product,
+// then E^1 ..), and what lies after them.
+template <typename T>
+size_t letters_smem(const Geometry& g, uint32_t block, int extras) {
+    const int M = g.depth - 1;
+    return (static_cast<size_t>(std::max(1, M)) * block * g.pw[M] + static_cast<size_t>(extras) * g.db[g.depth]) *
+           sizeof(T);
+}
 
 template <typename T, int W>
-__global__ void __launch_bounds__(1024) k_shuffle_letters_adjoint(Geometry G, PowerDiv pd, TArg<T> out, TArg<T> op,
-                                                                  TArg<T> arg, int64_t batch) {
+__global__ void __launch_bounds__(512) k_deal_adjoint(Geometry G, PowerDiv pd, int kind, TArg<T> out, TArg<T> op,
+                                                      TArg<T> arg, int64_t batch, T beta, uint32_t block) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* g = reinterpret_cast<T*>(smem_raw);  // degree N of the argument, then E^1, E^2, ...
-    const int D = G.depth, ohi = imin(out.hi, D);
-    const int phi = imin(op.hi, D), ahi = imin(arg.hi, D);
+    T* g = reinterpret_cast<T*>(smem_raw);
+    const int D = G.depth, ohi = imin(out.hi, D), phi = imin(op.hi, D), ahi = imin(arg.hi, D);
+    const uint32_t low = G.db[D];
+    T* P = g + static_cast<uint32_t>(imax(1, D - 1)) * block * G.pw[D - 1];  // the op below its top degree
+    T* sum_v = P + low;       // out[v]'s sums, and out[c v]'s: each updated once a block
+    T* sum_cv = sum_v + low;
+    const bool to_u = kind != static_cast<int>(ShuffleAdjKind::HalfR);
+    const bool to_v = kind != static_cast<int>(ShuffleAdjKind::HalfL);
     const uint32_t t0 = threadIdx.x, nt = blockDim.x, lane = t0 & 31u, warp = t0 >> 5, warps = nt >> 5;
-    T* P = g + static_cast<uint32_t>(D) * G.pw[D];  // the op
-    T* part = P + G.dim;                            // part[coefficient][warp]
     for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
         const T* A = arg.at(b);
+        const T* Pg = op.at(b);
         T* o = out.at(b);
-        if (op.lo <= phi) {
-            const T* src = op.at(b);
-            for (uint32_t i = G.db[op.lo] + t0; i < G.db[phi + 1]; i += nt) P[i] = src[i];
+        for (uint32_t i = t0; i < low; i += nt) {
+            sum_v[i] = sum_cv[i] = T(0);
+            P[i] = op.lo <= phi && i >= G.db[op.lo] && i < G.db[phi + 1] ? Pg[i] : T(0);
         }
-        // every coefficient of the output is one thread's for all N
-        for (int N = D; N >= 0; --N) {
-            const uint32_t size = G.pw[N];
-            const int kmax = imin(phi, N - out.lo), kmin = imax(op.lo, N - ohi);
-            const bool any = N >= arg.lo && N <= ahi && kmin <= kmax;
-            if (!any && N < D) continue;
-            if (any) {
-                for (uint32_t i = t0; i < size; i += nt) g[i] = A[G.db[N] + i];
+        __syncthreads();
+        bool top = false;  // the top degree's coefficients are written
+        for (int N = imin(ahi, D); N >= imax(arg.lo, 1); --N) {
+            const int M = N - 1, kcap = imin(M, imin(phi, M + 1 - out.lo));
+            if (kcap < 0) continue;
+            const uint32_t S = G.pw[M];
+            for (uint32_t c0 = 0; c0 < W; c0 += block) {
+                const uint32_t size = block * S;
+                for (uint32_t i = t0; i < size; i += nt) g[i] = A[G.db[N] + c0 * S + i];
                 __syncthreads();
-                for (int m = 1; m < N; ++m)
-                    for (int k = imin(m, kmax); k >= 1; --k) {
+                for (int m = 1; m < M; ++m)
+                    for (int k = imin(m, kcap); k >= 1; --k) {
                         T* E = g + static_cast<uint32_t>(k) * size;
                         const T* self = k == m ? g : E;
                         const T* prev = E - size;  // (k = 1: the argument)
-                        const int bl = m + 1 - k, R = N - m - 1;
 #pragma unroll 2
                         for (uint32_t i = t0; i < size; i += nt)
-                            E[i] = self[i] + prev[letter_past<W>(G, pd, i, bl, R)];
+                            E[i] = self[i] + prev[letter_back<W>(G, pd, i, m + 1 - k, k - 1)];
                         __syncthreads();
                     }
-            }
-            // out[N-k][v] += sum_u op[k][u] E^k[u, v]; N = D stores (zeros where it
-            // has no terms)
-            for (int q = out.lo; q <= ohi; ++q) {
-                const int k = N - q;
-                const bool terms = any && k >= kmin && k <= kmax;
-                if (!terms && N != D) continue;
-                const uint32_t wq = G.pw[q], wk = terms ? G.pw[k] : 0u;
-                const T* Pk = P + (terms ? G.db[k] : 0u);
-                const T* E = (k == 0 || k == N || !terms) ? g : g + static_cast<uint32_t>(k) * size;
-                if (wq >= 32u) {
-                    T* oq = o + G.db[q];
-                    for (uint32_t v = t0; v < wq; v += nt) {
-                        T acc = N == D ? T(0) : oq[v];
+                for (int k = 0; k <= kcap; ++k) {
+                    const int q = M - k;
+                    const bool in_u = to_u && k + 1 >= op.lo && k + 1 <= phi && q >= out.lo && q <= ohi;
+                    const bool in_v = to_v && k >= op.lo && k <= phi && q + 1 >= out.lo && q + 1 <= ohi;
+                    if (!in_u && !in_v) continue;
+                    const uint32_t wq = G.pw[q], wk = G.pw[k];
+                    const T* E = (k == 0 || k == M) ? g : g + static_cast<uint32_t>(k) * size;
+                    const T* Pu = k + 1 == D ? Pg + G.db[D] : P + G.db[k + 1];  // op[c u]
+                    const T* Pv = P + G.db[k];                                   // op[u]
+                    // (a warp's sums take five additions more; the barriers between the
+                    // blocks order the sums' updates, whichever thread makes them)
+                    if (wq >= 16u || wk < 64u) {
+                        for (uint32_t v = t0; v < wq; v += nt) {
+                            T s = T(0);
+                            for (uint32_t c = 0; c < block; ++c) {
+                                const T* row = E + (c * wq + v) * wk;
+                                const T* pc = Pu + (c0 + c) * wk;
+                                T d = T(0);
+                                if (in_u && in_v) {
 #pragma unroll 4
-                        for (uint32_t u = 0; u < wk; ++u) acc = fma(Pk[u], E[u * wq + v], acc);
-                        oq[v] = acc;
-                    }
-                } else {
-                    const uint32_t us = 32u / wq, u0 = lane / wq, v = lane - u0 * wq;
-                    T acc = T(0);
-                    if (u0 < us)
+                                    for (uint32_t u = 0; u < wk; ++u) {
+                                        const T e = row[u];
+                                        s = fma(pc[u], e, s);
+                                        d = fma(Pv[u], e, d);
+                                    }
+                                } else if (in_u) {
+#pragma unroll 4
+                                    for (uint32_t u = 0; u < wk; ++u) s = fma(pc[u], row[u], s);
+                                } else {
+#pragma unroll 4
+                                    for (uint32_t u = 0; u < wk; ++u) d = fma(Pv[u], row[u], d);
+                                }
+                                if (in_v) {
+                                    const uint32_t at = G.db[q + 1] + (c0 + c) * wq + v;
+                                    if (q + 1 == D) o[at] = d * beta;
+                                    else sum_cv[at] += d;
+                                }
+                            }
+                            if (in_u) sum_v[G.db[q] + v] += s;
+                        }
+                    } else {
+                        for (uint32_t v = warp; v < wq; v += warps) {
+                            T s = T(0);
+                            for (uint32_t c = 0; c < block; ++c) {
+                                const T* row = E + (c * wq + v) * wk;
+                                const T* pc = Pu + (c0 + c) * wk;
+                                T d = T(0);
 #pragma unroll 2
-                        for (uint32_t u = warp * us + u0; u < wk; u += us * warps) acc = fma(Pk[u], E[u * wq + v], acc);
-                    for (uint32_t off = wq; off < 32u; off *= 2u) {
-                        const T x = __shfl_down_sync(0xffffffffu, acc, off);
-                        if (lane + off < 32u) acc += x;
+                                for (uint32_t u = lane; u < wk; u += 32u) {
+                                    const T e = row[u];
+                                    if (in_u) s = fma(pc[u], e, s);
+                                    if (in_v) d = fma(Pv[u], e, d);
+                                }
+                                if (in_v) {
+#pragma unroll
+                                    for (uint32_t off = 16u; off > 0u; off /= 2u) d += __shfl_down_sync(0xffffffffu, d, off);
+                                    const uint32_t at = G.db[q + 1] + (c0 + c) * wq + v;
+                                    if (lane == 0) {
+                                        if (q + 1 == D) o[at] = d * beta;
+                                        else sum_cv[at] += d;
+                                    }
+                                }
+                            }
+                            if (in_u) {
+#pragma unroll
+                                for (uint32_t off = 16u; off > 0u; off /= 2u) s += __shfl_down_sync(0xffffffffu, s, off);
+                                if (lane == 0) sum_v[G.db[q] + v] += s;
+                            }
+                        }
                     }
-                    if (lane < wq) part[(G.db[q] + lane) * warps + warp] = acc;
+                    top = top || (in_v && q + 1 == D);
                 }
+                __syncthreads();
             }
-            __syncthreads();
-            // the narrow degrees' sums
-            for (uint32_t c = t0; c < kNarrow<W> && c < G.dim; c += nt) {
-                int q = 0;
-                while (c >= G.db[q + 1]) ++q;
-                const int k = N - q;
-                const bool terms = any && k >= kmin && k <= kmax;
-                if (q < out.lo || q > ohi || !(terms || N == D)) continue;
-                T acc = N == D ? T(0) : o[c];
-                const uint32_t used = terms ? warps : 0u;
-                for (uint32_t w = 0; w < used; ++w) acc += part[c * warps + w];
-                o[c] = acc;
-            }
-            __syncthreads();
         }
+        if (t0 == 0 && kind == static_cast<int>(ShuffleAdjKind::Shuffle) && arg.lo == 0 && ahi >= 0 && op.lo == 0 &&
+            phi >= 0 && out.lo == 0)
+            sum_v[0] = fma(P[0], A[0], sum_v[0]);
+        __syncthreads();
+        for (uint32_t i = G.db[out.lo] + t0; i < G.db[imin(ohi, D - 1) + 1]; i += nt) o[i] = (sum_v[i] + sum_cv[i]) * beta;
+        if (ohi == D && !top)
+            for (uint32_t i = low + t0; i < G.dim; i += nt) o[i] = T(0);
+        __syncthreads();
     }
 }
 
 template <typename T, int W>
-__global__ void __launch_bounds__(1024) k_shuffle_letters_product(Geometry G, PowerDiv pd, int kind, TArg<T> out,
-                                                                  TArg<T> add, TArg<T> lhs, TArg<T> rhs,
-                                                                  int64_t batch, T alpha, T beta) {
+__global__ void __launch_bounds__(512) k_deal_product(Geometry G, PowerDiv pd, int kind, TArg<T> out, TArg<T> add,
+                                                      TArg<T> lhs, TArg<T> rhs, int64_t batch, T alpha, T beta,
+                                                      uint32_t block) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* g = reinterpret_cast<T*>(smem_raw);  // degree N of the product, then E^1, E^2, ...
-    const int D = G.depth, ohi = imin(out.hi, D), lhi = imin(lhs.hi, D), rhi = imin(rhs.hi, D);
+    T* g = reinterpret_cast<T*>(smem_raw);
+    const int D = G.depth, ohi = imin(out.hi, D);
+    const uint32_t low = G.db[D];
+    T* sL = g + static_cast<uint32_t>(imax(1, D - 1)) * block * G.pw[D - 1];  // the factors below their top degree
+    T* sR = sL + low;
+    const bool both = kind != static_cast<int>(ShuffleKind::LeftHalf);
     const uint32_t t0 = threadIdx.x, nt = blockDim.x;
     for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
-        const T* L = lhs.at(b);
-        const T* Rp = rhs.at(b);
+        const T* Lg = lhs.at(b);
+        const T* Rg = rhs.at(b);
         T* o = out.at(b);
-        for (int N = ohi; N >= out.lo; --N) {
-            const uint32_t size = G.pw[N];
-            // the splits |u| = k of both ranges, and the arrays they reach
-            const int kmin = imax(imax(lhs.lo, N - rhi), 0), kmax = imin(imin(lhi, N - rhs.lo), N);
-            const int top = imin(kmax, N - 1);
-            for (uint32_t i = t0; i < size; i += nt) {
-                T v = T(0);
-                if (kmin <= 0 && kmax >= 0) v = L[0] * Rp[G.db[N] + i];
-                if (N > 0 && kmin <= N && kmax >= N) v = fma(L[G.db[N] + i], Rp[0], v);
-                g[i] = v;
-            }
-            for (int k = 1; k <= top; ++k) {
-                T* E = g + static_cast<uint32_t>(k) * size;
-                for (uint32_t i = t0; i < size; i += nt) {
-                    uint32_t u, v;
-                    pd.by[N - k].divmod(i, u, v);
-                    E[i] = k >= kmin ? L[G.db[k] + u] * Rp[G.db[N - k] + v] : T(0);
-                }
-            }
-            __syncthreads();
-            for (int m = N - 1; m >= 1; --m)
-                for (int k = 1; k <= imin(m, top); ++k) {
-                    const T* E = g + static_cast<uint32_t>(k) * size;
-                    T* prev = g + static_cast<uint32_t>(k - 1) * size;  // (k = 1: the product)
-                    const int bl = m + 1 - k, R = N - m - 1;
-                    if (k == m && k > 1) {
-                        // E^m ends here: it is the product's own share too
-#pragma unroll 2
-                        for (uint32_t i = t0; i < size; i += nt) {
-                            prev[i] += E[letter_back<W>(G, pd, i, bl, R)];
-                            g[i] += E[i];
-                        }
-                    } else if (k == m) {
-                        for (uint32_t i = t0; i < size; i += nt) g[i] += E[letter_back<W>(G, pd, i, bl, R)] + E[i];
-                    } else {
-#pragma unroll 2
-                        for (uint32_t i = t0; i < size; i += nt) prev[i] += E[letter_back<W>(G, pd, i, bl, R)];
-                    }
-                    __syncthreads();
-                }
-            T* oN = o + G.db[N];
-            const T* aN = kind == static_cast<int>(ShuffleKind::InplaceFma) ? oN
-                          : kind == static_cast<int>(ShuffleKind::Fma) && add.p && add.has(N) ? add.at(b) + G.db[N]
-                                                                                              : nullptr;
-            for (uint32_t i = t0; i < size; i += nt) {
-                T v = g[i] * beta;
-                if (aN) v = fma(alpha, aN[i], v);
-                oN[i] = v;
-            }
-            __syncthreads();
+        for (uint32_t i = t0; i < low; i += nt) {
+            sL[i] = Lg[i];
+            sR[i] = Rg[i];
         }
+        __syncthreads();
+        auto L = [&](int n, uint32_t i) -> T { return n < D ? sL[G.db[n] + i] : Lg[low + i]; };
+        auto R = [&](int n, uint32_t i) -> T { return n < D ? sR[G.db[n] + i] : Rg[low + i]; };
+        // the result of degree N, coefficient `at`, from its product
+        auto finish = [&](int N, uint32_t at, T v) {
+            v *= beta;
+            T* dst = o + G.db[N] + at;
+            if (kind == static_cast<int>(ShuffleKind::InplaceFma)) v = fma(alpha, *dst, v);
+            else if (kind == static_cast<int>(ShuffleKind::Fma) && add.p && add.has(N)) v = fma(alpha, add.at(b)[G.db[N] + at], v);
+            *dst = v;
+        };
+        for (int N = ohi; N >= imax(out.lo, 1); --N) {
+            const int M = N - 1;
+            const uint32_t S = G.pw[M];
+            for (uint32_t c0 = 0; c0 < W; c0 += block) {
+                const uint32_t size = block * S;
+                for (uint32_t i = t0; i < size; i += nt) {
+                    uint32_t c, j;
+                    pd.by[M].divmod(i, c, j);
+                    c += c0;
+                    T v = L(1, c) * R(M, j);  // k = 0
+                    if (both) v = fma(L(0, 0), R(N, c * S + j), v);
+                    if (M > 0) {  // k = M
+                        v = fma(L(N, c * S + j), R(0, 0), v);
+                        if (both) v = fma(L(M, j), R(1, c), v);
+                    }
+                    g[i] = v;
+                }
+                for (int k = 1; k < M; ++k) {
+                    T* E = g + static_cast<uint32_t>(k) * size;
+                    const T *Lc = sL + G.db[k + 1], *Lu = sL + G.db[k], *Rv = sR + G.db[M - k], *Rc = sR + G.db[M - k + 1];
+                    const uint32_t wk = G.pw[k], wv = G.pw[M - k];
+                    for (uint32_t i = t0; i < size; i += nt) {
+                        uint32_t t, c, u, v;
+                        pd.by[k].divmod(i, t, u);
+                        pd.by[M - k].divmod(t, c, v);
+                        c += c0;
+                        T e = Lc[c * wk + u] * Rv[v];
+                        if (both) e = fma(Lu[u], Rc[c * wv + v], e);
+                        E[i] = e;
+                    }
+                }
+                __syncthreads();
+                for (int m = M - 1; m >= 1; --m)
+                    for (int k = 1; k <= m; ++k) {
+                        const T* E = g + static_cast<uint32_t>(k) * size;
+                        T* prev = g + static_cast<uint32_t>(k - 1) * size;  // (k = 1: the product)
+                        const int bl = m + 1 - k, r = k - 1;
+                        if (k < m) {
+#pragma unroll 2
+                            for (uint32_t i = t0; i < size; i += nt) prev[i] += E[letter_past<W>(G, pd, i, bl, r)];
+                        } else if (k > 1) {  // E^m ends here: it is the product's own share too
+#pragma unroll 2
+                            for (uint32_t i = t0; i < size; i += nt) {
+                                prev[i] += E[letter_past<W>(G, pd, i, bl, r)];
+                                g[i] += E[i];
+                            }
+                        } else {
+                            for (uint32_t i = t0; i < size; i += nt) g[i] += E[letter_past<W>(G, pd, i, bl, r)] + E[i];
+                        }
+                        __syncthreads();
+                    }
+                for (uint32_t i = t0; i < size; i += nt) finish(N, c0 * S + i, g[i]);
+                __syncthreads();
+            }
+        }
+        if (out.lo == 0 && t0 == 0) {
+            if (both) finish(0, 0, L(0, 0) * R(0, 0));
+            else o[0] = T(0);
+        }
+        __syncthreads();
     }
-}
-
-template <typename T>
-size_t letters_smem(const Geometry& g) {
-    return static_cast<size_t>(std::max(1, g.depth)) * g.pw[g.depth] * sizeof(T);
-}
-
-template <typename T>
-size_t letters_adjoint_smem(const Geometry& g, int threads) {
-    return letters_smem<T>(g) + (g.dim + 40 * static_cast<size_t>(threads / 32)) * sizeof(T);
 }
 
 template <typename T>
@@ -234,12 +301,17 @@ bool apart(const Geometry& g, const TArg<T>& a, const TArg<T>& b, int64_t batch)
     return end(a) <= begin(b) || end(b) <= begin(a);
 }
 
-// Four words of the widest degree a thread; an SM's worth of threads where one
-// CTA fits it.
-int letters_threads(const Geometry& g, size_t smem) {
-    const int most = smem > 110 * 1024 ? 1024 : smem > 72 * 1024 ? 512 : 256;
-    return std::max(32, std::min(most, static_cast<int>((g.pw[g.depth] / 4 + 31) / 32 * 32)));
+// First letters at a time, shared memory and threads (four words each) of a
+// launch: all first letters where six CTAs still fit an SM, else one.
+template <typename T>
+void letters_shape(const Geometry& g, int extras, uint32_t& block, size_t& smem, int& threads) {
+    block = static_cast<uint32_t>(g.width);
+    if (letters_smem<T>(g, block, extras) > 36 * 1024) block = 1;
+    smem = letters_smem<T>(g, block, extras);
+    const int most = smem > 100 * 1024 ? 512 : 256;
+    threads = std::max(32, std::min(most, static_cast<int>((block * g.pw[g.depth - 1] / 4 + 31) / 32 * 32)));
 }
+constexpr int kAdjointExtras = 3, kProductExtras = 2;
 
 PowerDiv power_div(const Geometry& g) {
     PowerDiv pd;
@@ -247,30 +319,47 @@ PowerDiv power_div(const Geometry& g) {
     return pd;
 }
 
-// Where dealing letters is the faster way: the steps are barrier-separated, so
-// three CTAs an SM are wanted (all in FP32 that fits), or operations that are
-// three times fewer at least -- 2^D against D (D+1) / 2.  With one CTA an SM W5 D5
-// FP64 took 1 007 us (product) and 1 500 (adjoint), the subsets 832 and 974.
 template <typename T>
-bool letters_fit(const Geometry& g, const DeviceInfo& dev) {
-    const int D = g.depth;
-    const size_t smem = letters_smem<T>(g);
-    if (!column_width(g.width) || D < 3 || D > kLettersMaxDepth) return false;
-    if (smem > std::min(kLettersSmemLimit, static_cast<size_t>(dev.max_smem_optin))) return false;
-    return smem <= 66 * 1024 || (1u << D) >= 3u * static_cast<uint32_t>(D * (D + 1) / 2);
+bool letters_fit(const Geometry& g, const DeviceInfo& dev, int extras) {
+    if (!column_width(g.width) || g.depth < 3 || g.depth > kLettersMaxDepth) return false;
+    uint32_t block;
+    size_t smem;
+    int threads;
+    letters_shape<T>(g, extras, block, smem, threads);
+    return smem <= std::min(kLettersSmemLimit, static_cast<size_t>(dev.max_smem_optin));
+}
+
+// Where dealing letters is the faster way.  From degree 6 on it has a third of the
+// operations or fewer.  Below, FP32 gains from its plain loops, except where a
+// half-shuffle adjoint of a wide tensor waits at its barriers (W6 D5 left 634 us,
+// 360 by subsets); FP64 only where most of the operations are additions, the
+// products (W4 D4 16.5 -> 13.6; but W8 D4 611, 558 by subsets; left_hs_mul W5 D5
+// 546, 467 by subsets; st_adj_mul W5 D5 1263, 974 by subsets).
+template <typename T>
+bool letters_pay(const Geometry& g, ShuffleKind kind) {
+    if (std::is_same<T, float>::value || g.depth >= 6) return true;
+    if (kind == ShuffleKind::LeftHalf) return g.dim <= 1200;
+    return g.depth >= 4 && (g.width <= 6 || g.depth >= 5);
+}
+template <typename T>
+bool letters_pay(const Geometry& g, ShuffleAdjKind kind) {
+    if (g.depth >= 6) return true;
+    if (std::is_same<T, double>::value) return false;
+    if (kind == ShuffleAdjKind::HalfL) return g.dim <= 1200;
+    return kind == ShuffleAdjKind::Shuffle || (g.depth >= 4 && g.dim <= 5000);
 }
 
 }  // namespace
 
 // Operands are read as the result is written: the output must lie apart from
-// both (the added term may be the output itself).
+// both (the added term may be the output itself).  The product's factors are
+// whole tensors (degrees that a view lacks would be multiplied as zeros).
 template <typename T>
 bool shuffle_letters_product_fits(const Geometry& g, const DeviceInfo& dev, ShuffleKind kind, const TArg<T>& out,
                                   const TArg<T>& add, const TArg<T>& lhs, const TArg<T>& rhs, int64_t batch) {
     const bool same = add.p == out.p && (batch == 1 || add.stride == out.stride);
-    // (degree 3 in FP64, 9 operations against 8: W4 D3 23 us, 20 by subsets)
-    if (std::is_same<T, double>::value && g.depth < 4) return false;
-    return kind != ShuffleKind::LeftHalf && out.lo <= out.hi && letters_fit<T>(g, dev) && apart(g, out, lhs, batch) &&
+    const bool whole = lhs.lo == 0 && rhs.lo == 0 && lhs.hi >= g.depth && rhs.hi >= g.depth;
+    return whole && out.lo <= out.hi && letters_pay<T>(g, kind) && letters_fit<T>(g, dev, kProductExtras) && apart(g, out, lhs, batch) &&
            apart(g, out, rhs, batch) && (kind != ShuffleKind::Fma || same || apart(g, out, add, batch));
 }
 
@@ -278,32 +367,37 @@ template <typename T>
 cudaError_t launch_shuffle_letters_product(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, ShuffleKind kind,
                                            TArg<T> out, TArg<T> add, TArg<T> lhs, TArg<T> rhs, int64_t batch,
                                            double alpha, double beta) {
-    const size_t smem = letters_smem<T>(g);
+    uint32_t block;
+    size_t smem;
+    int threads;
+    letters_shape<T>(g, kProductExtras, block, smem, threads);
     return with_width(g.width, [&](auto w) {
         constexpr int W = decltype(w)::value;
-        return run_column<&k_shuffle_letters_product<T, W>>(dev, s, letters_threads(g, smem), smem, batch, g,
-                                                            power_div(g), static_cast<int>(kind), out, add, lhs, rhs,
-                                                            batch, static_cast<T>(alpha), static_cast<T>(beta));
+        return run_column<&k_deal_product<T, W>>(dev, s, threads, smem, batch, g, power_div(g), static_cast<int>(kind),
+                                                 out, add, lhs, rhs, batch, static_cast<T>(alpha),
+                                                 static_cast<T>(beta), block);
     });
 }
 
 template <typename T>
 bool shuffle_letters_adjoint_fits(const Geometry& g, const DeviceInfo& dev, ShuffleAdjKind kind, const TArg<T>& out,
                                   const TArg<T>& op, const TArg<T>& arg, int64_t batch) {
-    return kind == ShuffleAdjKind::Shuffle && out.lo <= out.hi && letters_fit<T>(g, dev) &&
-           letters_adjoint_smem<T>(g, letters_threads(g, letters_smem<T>(g))) <= kLettersSmemLimit &&
-           apart(g, out, op, batch) && apart(g, out, arg, batch);
+    return out.lo <= out.hi && letters_pay<T>(g, kind) && letters_fit<T>(g, dev, kAdjointExtras) && apart(g, out, op, batch) &&
+           apart(g, out, arg, batch);
 }
 
 template <typename T>
-cudaError_t launch_shuffle_letters_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out,
-                                           TArg<T> op, TArg<T> arg, int64_t batch) {
-    const int threads = letters_threads(g, letters_smem<T>(g));
-    const size_t smem = letters_adjoint_smem<T>(g, threads);
+cudaError_t launch_shuffle_letters_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s,
+                                           ShuffleAdjKind kind, TArg<T> out, TArg<T> op, TArg<T> arg, int64_t batch,
+                                           double beta) {
+    uint32_t block;
+    size_t smem;
+    int threads;
+    letters_shape<T>(g, kAdjointExtras, block, smem, threads);
     return with_width(g.width, [&](auto w) {
         constexpr int W = decltype(w)::value;
-        return run_column<&k_shuffle_letters_adjoint<T, W>>(dev, s, threads, smem, batch, g, power_div(g), out, op, arg,
-                                                            batch);
+        return run_column<&k_deal_adjoint<T, W>>(dev, s, threads, smem, batch, g, power_div(g), static_cast<int>(kind),
+                                                 out, op, arg, batch, static_cast<T>(beta), block);
     });
 }
 
@@ -315,8 +409,8 @@ cudaError_t launch_shuffle_letters_adjoint(const Geometry& g, const DeviceInfo& 
                                                            int64_t, double, double);                                \
     template bool shuffle_letters_adjoint_fits<T>(const Geometry&, const DeviceInfo&, ShuffleAdjKind,               \
                                                   const TArg<T>&, const TArg<T>&, const TArg<T>&, int64_t);         \
-    template cudaError_t launch_shuffle_letters_adjoint<T>(const Geometry&, const DeviceInfo&, cudaStream_t, TArg<T>, \
-                                                           TArg<T>, TArg<T>, int64_t);
+    template cudaError_t launch_shuffle_letters_adjoint<T>(const Geometry&, const DeviceInfo&, cudaStream_t,        \
+                                                           ShuffleAdjKind, TArg<T>, TArg<T>, TArg<T>, int64_t, double);
 
 RPP_GB_INSTANTIATE_LETTERS(float)
 RPP_GB_INSTANTIATE_LETTERS(double)

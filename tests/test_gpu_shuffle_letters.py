@@ -1,4 +1,4 @@
-"""The shuffle product and its adjoint a letter at a time
+"""The shuffle and half-shuffle products and their adjoints a letter at a time
 (csrc/shuffle_letters.cu) against the subset sums in numpy, FP64: strided and
 unaligned rows, degree ranges, the in-place and fused forms, and outputs that
 alias an operand (which take the general kernel)."""
@@ -14,35 +14,41 @@ pytestmark = pytest.mark.gpu
 pkg = importlib.import_module("rough-path-primitives_gb300")
 from test_gpu_column import EPS, Rows, check, restrict, starts  # noqa: E402
 
-SHAPES = [(2, 3, 5), (2, 7, 3), (2, 10, 2), (3, 4, 40), (3, 5, 3), (4, 3, 600), (4, 4, 5), (5, 3, 33), (5, 4, 3), (6, 3, 7),
-          (7, 3, 3), (8, 3, 5)]
+SHAPES = [(2, 3, 5), (2, 6, 40), (2, 7, 3), (2, 10, 2), (3, 4, 40), (3, 5, 3), (4, 3, 600), (4, 4, 5), (5, 3, 33), (5, 4, 3), (6, 3, 7),
+          (3, 6, 3), (7, 3, 3), (8, 3, 5)]
 
 
-def splits(n, k):
-    """Axis orders that gather a word's letters at k places in front, the others behind."""
+def splits(n, k, half=False):
+    """Axis orders that gather a word's letters at k places (`half`: the first
+    among them) in front, the others behind."""
     for places in itertools.combinations(range(n), k):
-        yield list(places) + [i for i in range(n) if i not in places]
+        if not half or 0 in places:
+            yield list(places) + [i for i in range(n) if i not in places]
 
 
-def shuffle(x, y, W, D):
+def shuffle(x, y, W, D, half=False):
     db, out = starts(W, D), np.zeros_like(x)
-    for n in range(D + 1):
+    for n in range(1 if half else 0, D + 1):
         for k in range(n + 1):
             both = (x[:, db[k]:db[k + 1], None] * y[:, None, db[n - k]:db[n - k + 1]]).reshape([len(x)] + [W] * n)
-            for order in splits(n, k):
+            for order in splits(n, k, half):
                 back = np.argsort(order)
                 out[:, db[n]:db[n + 1]] += both.transpose([0] + [i + 1 for i in back]).reshape(len(x), -1)
     return out
 
 
-def adjoint(op, arg, W, D):
+def adjoint(op, arg, W, D, half=False, first=False):
+    """The gradient of <arg, op sh y> in y, or with `first` of <arg, x sh op> in x."""
     db, out = starts(W, D), np.zeros_like(arg)
-    for n in range(D + 1):
+    for n in range(1 if half else 0, D + 1):
         g = arg[:, db[n]:db[n + 1]].reshape([len(arg)] + [W] * n)
         for k in range(n + 1):
-            for order in splits(n, k):
+            for order in splits(n, k, half):
                 m = g.transpose([0] + [i + 1 for i in order]).reshape(len(arg), W ** k, W ** (n - k))
-                out[:, db[n - k]:db[n - k + 1]] += (op[:, None, db[k]:db[k + 1]] @ m)[:, 0]
+                if first:
+                    out[:, db[k]:db[k + 1]] += (m @ op[:, db[n - k]:db[n - k + 1], None])[:, :, 0]
+                else:
+                    out[:, db[n - k]:db[n - k + 1]] += (op[:, None, db[k]:db[k + 1]] @ m)[:, 0]
     return out
 
 
@@ -76,6 +82,15 @@ def test_products_and_adjoint_by_letters(W, D, B, dtype):
             before = out.host()
             assert pkg.st_adj_mul(st, None, out.view(*ro), x.view(*rx), y.view(*ry), basis, B)
             check(out.host(), before, adjoint(hx, hy, W, D), W, D, ro, tol_adjoint)
+            before = out.host()
+            assert pkg.left_hs_mul(st, None, out.view(*ro), x.view(*rx), y.view(*ry), basis, B, -0.5)
+            check(out.host(), before, -0.5 * shuffle(hx, hy, W, D, True), W, D, ro, tol)
+            before = out.host()
+            assert pkg.left_hs_adj_lmul(st, None, out.view(*ro), x.view(*rx), y.view(*ry), basis, B, -0.5)
+            check(out.host(), before, -0.5 * adjoint(hx, hy, W, D, True), W, D, ro, tol_adjoint)
+            before = out.host()
+            assert pkg.left_hs_adj_rmul(st, None, out.view(*ro), x.view(*rx), y.view(*ry), basis, B, -0.5)
+            check(out.host(), before, -0.5 * adjoint(hy, hx, W, D, True, True), W, D, ro, tol_adjoint)
         # the result over an operand
         want = shuffle(x.host(), y.host(), W, D)
         assert pkg.st_mul(st, None, x.view(), x.view(), y.view(), basis, B)
