@@ -16,10 +16,12 @@
 // is what FP32 gains from: the general kernel spends ten instructions a
 // multiply-add and two CTA barriers a degree.  Bound by instruction issue in FP32
 // (0.76 instructions a clock and scheduler at W5 D5), by the pipe in FP64.
-// Left / right, general kernel -> this: FP32 W5 D5 batch 4096 112 -> 78 / 119 ->
-// 106 us, W8 D4 111 -> 79 / 117 -> 81, W2 D12 batch 2048 183 -> 118 / 211 -> 152;
-// FP64 W5 D5 221 -> 203 / 233 -> 211, W2 D8 99 -> 47 / 137 -> 73, W2 D12 547 -> 428 /
-// 591 -> 502.
+// FP32 sums are formed in short blocks: shorter chains of dependent additions
+// (left W5 D5 78 -> 68 us) and a smaller rounding error.
+// Left / right, general kernel -> this: FP32 W5 D5 batch 4096 112 -> 68 / 119 ->
+// 75 us, W8 D4 111 -> 68 / 117 -> 81, W2 D12 batch 2048 183 -> 111 / 211 -> 152;
+// FP64 W5 D5 221 -> 204 / 233 -> 211, W2 D8 99 -> 47 / 137 -> 73, W2 D12 547 -> 430 /
+// 591 -> 503.
 #include <algorithm>
 #include <type_traits>
 
@@ -61,6 +63,27 @@ AdjointTasks adjoint_tasks(const Geometry& g, bool left, bool fp64, int olo, int
     }
     k.start[g.depth + 1] = at;
     return k;
+}
+
+// acc + sum over i < n, in steps of `step` from `first`, of x[i] y[i ys].  FP32 sums
+// blocks of eight first: a chain of hundreds of additions would double the
+// rounding error of the general kernel's shorter ones.
+template <typename T>
+__device__ __forceinline__ T dot(const T* x, const T* y, uint32_t first, uint32_t n, uint32_t step, uint32_t ys, T acc) {
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll 4
+        for (uint32_t i = first; i < n; i += step) acc = fma(x[i], y[i * ys], acc);
+    } else {
+        uint32_t i = first;
+        for (; i + 7u * step < n; i += 8u * step) {
+            T part = x[i] * y[i * ys];
+#pragma unroll
+            for (uint32_t r = 1; r < 8; ++r) part = fma(x[i + r * step], y[(i + r * step) * ys], part);
+            acc += part;
+        }
+        for (; i < n; i += step) acc = fma(x[i], y[i * ys], acc);
+    }
+    return acc;
 }
 
 template <typename T, int W, bool Left>
@@ -110,9 +133,7 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                         for (int p = pmin; p <= pmax; ++p) {
                             const T* Pp = P + G.db[p];
                             const T* Ap = A + G.db[m + p] + j;
-                            const uint32_t wp = G.pw[p];
-#pragma unroll 4
-                            for (uint32_t u = u0; u < wp; u += us) acc = fma(Pp[u], Ap[u * wm], acc);
+                            acc = dot(Pp, Ap, u0, G.pw[p], us, wm, acc);
                         }
                     for (uint32_t off = wm; off < 32u; off *= 2u) {
                         const T x = __shfl_down_sync(0xffffffffu, acc, off);
@@ -158,23 +179,34 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                     const uint32_t wp = G.pw[p];
                     if constexpr (Left) {
                         const T* Ap = A + G.db[m + p] + j;
-                        for (uint32_t u = 0; u < wp; u += W, Pp += W, Ap += W * wm)
+                        for (uint32_t u = 0; u < wp; u += W, Pp += W, Ap += W * wm) {
+                            T part = sizeof(T) == 4 ? T(0) : acc;  // (FP32: blocks first, as in dot())
 #pragma unroll
-                            for (int a = 0; a < W; ++a) acc = fma(Pp[a], Ap[a * wm], acc);
+                            for (int a = 0; a < W; ++a) part = fma(Pp[a], Ap[a * wm], part);
+                            acc = sizeof(T) == 4 ? acc + part : part;
+                        }
                     } else {
                         const T* Ap = A + G.db[m + p] + j * wp;
                         if constexpr ((W & (W - 1)) == 0) {
                             constexpr uint32_t lanes = 128u / sizeof(T);  // of one pass over the banks
                             uint32_t v = (wp <= lanes ? j * wp / lanes : j) & (wp - 1u);
-#pragma unroll 4
-                            for (uint32_t i = 0; i < wp; ++i) {
-                                acc = fma(Pp[v], Ap[v], acc);
-                                v = (v + 1u) & (wp - 1u);
+                            constexpr uint32_t block = W < 4 ? 4u : W;  // divides wp = W^p, p >= 2
+                            for (uint32_t i = 0; i < wp; i += block) {
+                                T part = sizeof(T) == 4 ? T(0) : acc;
+#pragma unroll
+                                for (uint32_t a = 0; a < block; ++a) {
+                                    part = fma(Pp[v], Ap[v], part);
+                                    v = (v + 1u) & (wp - 1u);
+                                }
+                                acc = sizeof(T) == 4 ? acc + part : part;
                             }
                         } else {
-                            for (uint32_t v = 0; v < wp; v += W)
+                            for (uint32_t v = 0; v < wp; v += W) {
+                                T part = sizeof(T) == 4 ? T(0) : acc;
 #pragma unroll
-                                for (int a = 0; a < W; ++a) acc = fma(Pp[v + a], Ap[v + a], acc);
+                                for (int a = 0; a < W; ++a) part = fma(Pp[v + a], Ap[v + a], part);
+                                acc = sizeof(T) == 4 ? acc + part : part;
+                            }
                         }
                     }
                 }
