@@ -69,8 +69,13 @@ size_t horner_smem(const Geometry& g, bool multiplier) {
 }  // namespace
 
 template <typename T>
-bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out) {
+bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out,
+                        const TArg<T>& x) {
     const bool fm = kind == IntermediateKind::FMExp;
+    // (an exponent without degree one leaves degrees of its exponential that have no
+    // terms: the general kernel skips them, a product with their zeros would turn
+    // the multiplier's infinities into NaN)
+    if (fm && (x.lo > 1 || x.hi < 1)) return false;
     return out.lo <= out.hi && (fm || out.lo == 0) && horner_fits(g, dev, horner_smem<T>(g, fm));
 }
 
@@ -86,7 +91,8 @@ cudaError_t launch_column_horner(const Geometry& g, const DeviceInfo& dev, cudaS
 }
 
 #define RPP_GB_INSTANTIATE_HORNER(T)                                                                                \
-    template bool column_horner_fits<T>(const Geometry&, const DeviceInfo&, IntermediateKind, const TArg<T>&);      \
+    template bool column_horner_fits<T>(const Geometry&, const DeviceInfo&, IntermediateKind, const TArg<T>&,       \
+                                        const TArg<T>&);                                                        \
     template cudaError_t launch_column_horner<T>(const Geometry&, const DeviceInfo&, cudaStream_t, IntermediateKind, \
                                                  TArg<T>, TArg<T>, TArg<T>, int64_t);
 

@@ -435,7 +435,7 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
     if (kind != IntermediateKind::Log && chen_step_fits<T>(g, dev, out, x))
         return launch_chen_step<T>(g, dev, s, out, kind == IntermediateKind::FMExp ? m : TArg<T>{nullptr, 0, 1, 0}, x,
                                    batch, kind == IntermediateKind::Exp && out.lo == 0);
-    if (column_horner_fits<T>(g, dev, kind, out)) return launch_column_horner<T>(g, dev, s, kind, out, x, m, batch);
+    if (column_horner_fits<T>(g, dev, kind, out, x)) return launch_column_horner<T>(g, dev, s, kind, out, x, m, batch);
     constexpr auto kernel = k_intermediate<T>;
     cudaError_t err = allow_large_smem<kernel>(dev);
     if (err != cudaSuccess) return err;

@@ -116,7 +116,9 @@ cudaError_t launch_column_log_to_lie(const Geometry& g, const DeviceInfo& dev, c
 
 template <typename T>
 bool column_lie_exp_fits(const Geometry& g, const DeviceInfo& dev, const CsrDevice& m, const TArg<T>& out,
-                         bool multiplier) {
+                         bool multiplier, int lo, int hi) {
+    // (an exponent without degree one: see column_horner_fits)
+    if (multiplier && (lo > 1 || hi < 1)) return false;
     // (the smallest FP64 tensors, one warp each, gain nothing: W4 D3 37 us, 35 with the general kernel)
     if (std::is_same<T, double>::value && g.dim < 128) return false;
     return out.lo <= out.hi && (multiplier || out.lo == 0) && m.cols_dim <= static_cast<int64_t>(g.dim) &&
@@ -142,7 +144,8 @@ cudaError_t launch_column_lie_exp(const Geometry& g, const DeviceInfo& dev, cuda
     template cudaError_t launch_column_log_to_lie<T>(const Geometry&, const DeviceInfo&, cudaStream_t,              \
                                                      const CsrDevice&, TArg<T>, int, T*, int64_t, int64_t, int64_t, \
                                                      double);                                                       \
-    template bool column_lie_exp_fits<T>(const Geometry&, const DeviceInfo&, const CsrDevice&, const TArg<T>&, bool); \
+    template bool column_lie_exp_fits<T>(const Geometry&, const DeviceInfo&, const CsrDevice&, const TArg<T>&, bool,  \
+                                         int, int);                                                                   \
     template cudaError_t launch_column_lie_exp<T>(const Geometry&, const DeviceInfo&, cudaStream_t, const CsrDevice&, \
                                                   const T*, int64_t, int, int, TArg<T>, TArg<T>, int64_t, double);
 

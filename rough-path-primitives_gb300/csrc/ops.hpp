@@ -49,7 +49,8 @@ cudaError_t launch_chen_step(const Geometry& g, const DeviceInfo& dev, cudaStrea
 
 // exp / log / fmexp on columns of coefficients (widths 2..8, ft_horner.cu).
 template <typename T>
-bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out);
+bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out,
+                        const TArg<T>& x);
 template <typename T>
 cudaError_t launch_column_horner(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, IntermediateKind kind,
                                  TArg<T> out, TArg<T> x, TArg<T> m, int64_t batch);
@@ -202,7 +203,7 @@ cudaError_t launch_column_log_to_lie(const Geometry& g, const DeviceInfo& dev, c
                                      double alpha);
 template <typename T>
 bool column_lie_exp_fits(const Geometry& g, const DeviceInfo& dev, const CsrDevice& m, const TArg<T>& out,
-                         bool multiplier);
+                         bool multiplier, int lo, int hi);
 template <typename T>
 cudaError_t launch_column_lie_exp(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const CsrDevice& m,
                                   const T* lie, int64_t lie_stride, int lo, int hi, TArg<T> out, TArg<T> mult,

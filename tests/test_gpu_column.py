@@ -179,6 +179,21 @@ def test_horner_in_columns(W, D, B, dtype):
             check(out.host(), before, product(held, exp, W, D), W, D, ro, tol * (D + 1))
 
 
+@pytest.mark.parametrize("W,D", [(2, 5), (5, 3)])
+@pytest.mark.parametrize("rx", [(2, 3), (0, 0)])
+def test_exponent_without_degree_one_leaves_infinities_alone(W, D, rx):
+    # degrees of the exponential without terms take no part: M (x) exp(X) keeps
+    # M's degree 1 (and all of M where X has no terms), whatever its degree 0 holds
+    rng = np.random.default_rng(W)
+    st, basis, db = pkg.GB300Strategy(torch.float64), pkg.TensorBasis(W, D), starts(W, D)
+    out, x, m = (Rows(rng, torch.float64, W, D, 2, 0, 0, 0.25) for _ in range(3))
+    m.buf.view(2, -1)[:, 0] = float("inf")
+    assert pkg.ft_fmexp(st, None, out.view(0, D), m.view(0, D), x.view(*rx), basis, 2)
+    kept = int(db[2]) if rx[0] == 2 else int(db[-1])
+    # (scaled by D! and back: a rounding a round)
+    assert np.allclose(out.host()[:, :kept], m.host()[:, :kept], rtol=4 * D * EPS[torch.float64], atol=0)
+
+
 def adjoint(p, a, W, D, left):
     """out[m] = sum over p of the op's degree p against the argument's degree m + p."""
     db, out = starts(W, D), np.zeros_like(a)
