@@ -432,9 +432,14 @@ int rpp_gb_signature_static_scratch(const rpp_gb_plan* plan, rpp_gb_stream strea
  * final signatures, each holding less shared memory per CTA) on the caller's
  * own inputs, times each with CUDA events on `stream`, and records the
  * fastest for this (device, width, depth, dtype, outputs requested, ragged or
- * not); later rpp_gb_signature calls with that key use it.  Synchronises the
- * stream (not capturable); leaves the chosen schedule's outputs in sig/grad.
- * *threads and *ms (may be NULL) receive the choice and its time per call:
+ * not); later rpp_gb_signature calls with that key use it -- unless the form
+ * that a call without a schedule takes, which is timed beside them, is as fast:
+ * later calls then go on taking that form, chosen for their own batch.
+ * Synchronises the stream (not capturable); leaves the outputs of what later
+ * calls run in sig/grad.  *ms (may be NULL) receives the time per call of what
+ * later calls with these arguments run (paths that they cut in time, whatever
+ * is recorded, included), *threads (may be NULL) the fastest of the schedules
+ * tried, for pinning; the allocation-free and the grouped entry take that one:
  * threads per CTA in bits 0-9 of *threads, the cap on CTAs per SM (0 = none)
  * in bits 10-13, bit 14 set for the two-launch form, bit 15 set when its
  * forward launch (or a forward-only call) keeps the top level in the output

@@ -767,8 +767,9 @@ def exp_letter_vjp(strategy, config, cotangent, x, dx, basis, num_batches, *, co
 def signature_tune(strategy, config, increments, basis, num_batches, *, length=None, offsets=None, out=None,
                    out_stride=None, seed=None, seed_stride=None, grad=None):
     """Autotune the signature schedule on these inputs (rpp_gb_signature_tune);
-    returns (Error, threads per CTA chosen, ms per launch).  Later ``signature``
-    calls of the same shape use the choice."""
+    returns (Error, the fastest schedule tried, ms per call of later calls).  Later
+    ``signature`` calls of the same shape use that schedule, or go on without one
+    where the form they take by themselves is as fast."""
     _check_batches(strategy, *(TensorBatch(t, 0, 0, 0) for t in (increments, out, seed, grad) if t is not None))
     dim = basis.size()
     lib = _lib.load()

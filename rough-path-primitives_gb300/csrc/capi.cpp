@@ -273,8 +273,8 @@ int run_helper_any(const rpp_gb_plan* plan, rpp_gb_stream stream, int32_t dtype,
     });
 }
 
-// Schedules chosen by rpp_gb_signature_tune, keyed by the call's shape:
-// (device, width, depth, dtype, mode, ragged).  Read by every signature call.
+// What rpp_gb_signature_tune found, keyed by the call's shape: (device, width,
+// depth, dtype, mode, ragged).  Read by every signature call.
 struct ScheduleKey {
     int device, width, depth, dtype, mode, ragged;
     bool operator<(const ScheduleKey& o) const {
@@ -282,8 +282,12 @@ struct ScheduleKey {
                std::tie(o.device, o.width, o.depth, o.dtype, o.mode, o.ragged);
     }
 };
+struct Tuned {
+    int schedule = 0;        // the fastest explicit one (0: never tuned)
+    bool rule_wins = false;  // the form chosen by the rule on shape and batch is as fast
+};
 std::mutex g_schedule_lock;
-std::map<ScheduleKey, int> g_schedules;
+std::map<ScheduleKey, Tuned> g_schedules;
 
 ScheduleKey schedule_key(const rpp_gb_plan* plan, int32_t dtype, bool forward, const void* sig, const void* seed,
                          const int64_t* offsets) {
@@ -292,11 +296,14 @@ ScheduleKey schedule_key(const rpp_gb_plan* plan, int32_t dtype, bool forward, c
                        offsets != nullptr ? 1 : 0};
 }
 
-int scheduled_threads(const ScheduleKey& key) {
+Tuned tuned(const ScheduleKey& key) {
     std::lock_guard<std::mutex> guard(g_schedule_lock);
     auto it = g_schedules.find(key);
-    return it == g_schedules.end() ? 0 : it->second;
+    return it == g_schedules.end() ? Tuned{} : it->second;
 }
+
+// For the entries that always run an explicit schedule where there is one.
+int scheduled_threads(const ScheduleKey& key) { return tuned(key).schedule; }
 
 template <typename T>
 int check_signature_args(const rpp_gb_plan* plan, const void* incr, const int64_t* offsets, int64_t length,
@@ -329,7 +336,10 @@ int run_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const 
     // an explicit schedule runs the paths whole; otherwise few long paths may
     // be cut in time, whatever schedule is recorded for whole paths
     if (threads >= 0) whole_batch = -1;
-    if (threads < 0) threads = scheduled_threads(schedule_key(plan, dtype, forward, sig, seed, offsets));
+    if (threads < 0) {
+        const Tuned found = tuned(schedule_key(plan, dtype, forward, sig, seed, offsets));
+        threads = found.rule_wins ? 0 : found.schedule;
+    }
     rpp_gb::PathBatch paths{offsets, length, batch};
     return cuda_status(rpp_gb::launch_signature<T>(plan->geometry, plan->device, s, static_cast<const T*>(incr),
                                                    paths, static_cast<T*>(sig), sig_stride,
@@ -342,7 +352,10 @@ int run_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const 
 // CTAs per SM: see launch_width) on the caller's own inputs (one warm-up and
 // two timed launches each, CUDA events on `s`), keep the fastest.  Candidates
 // that cannot launch for this shape, or whose cap would not lower the
-// residency, are skipped.
+// residency, are skipped.  The form of a call without a schedule (threads 0)
+// is timed beside them: the rule picks CTA sizes, and pairs of them, that the
+// list does not hold (W4 D4 FP64, 4 096 x 16 forward: 83 us, where 128 threads
+// take 146), and keeps adapting to the batch.
 template <typename T>
 int tune_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const void* incr, const int64_t* offsets,
                    int64_t length, int64_t batch, void* sig, int64_t sig_stride, const void* seed,
@@ -466,31 +479,39 @@ int tune_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const
                 try_candidate(base[k] | rpp_gb::kScheduleMergedReverse);
     }
     // Near-ties are decided by noise in a single timing: time the three
-    // fastest once more and keep the best total of both timings.
-    if (top[1].second != 0) {
-        float best_total = 0.f;
-        for (const auto& c : top) {
-            float ms = 0.f;
-            if (c.second == 0 || !time_candidate(c.second, ms)) continue;
-            if (best_total == 0.f || c.first + ms < best_total) {
-                best_total = c.first + ms;
-                best = c.second;
-                best_ms = best_total / 2.f;
-            }
+    // fastest once more and keep the best total of both timings; the same for
+    // the form of a call without a schedule.
+    float best_total = 0.f;
+    for (const auto& c : top) {
+        float ms = 0.f;
+        if (c.second == 0 || !time_candidate(c.second, ms)) continue;
+        if (best_total == 0.f || c.first + ms < best_total) {
+            best_total = c.first + ms;
+            best = c.second;
         }
     }
+    float rule_first = 0.f, rule_again = 0.f;
+    const bool rule_wins = time_candidate(0, rule_first) && time_candidate(0, rule_again) && best_total > 0.f &&
+                           rule_first + rule_again <= best_total;
+    if (rule_wins) best_total = rule_first + rule_again;
+    best_ms = best_total / 4.f;
+    // paths that later calls cut in time: what these take, whatever is recorded
+    float cut_ms = 0.f;
+    if (!offsets && rpp_gb::signature_chunks<T>(geo, plan->device, batch, length, grad != nullptr) > 1 &&
+        time_candidate(-1, cut_ms))
+        best_ms = cut_ms / 2.f;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (best == 0) return fail(RPP_GB_NOT_IMPLEMENTED, "no signature schedule can launch for this shape");
     {
         std::lock_guard<std::mutex> guard(g_schedule_lock);
-        g_schedules[schedule_key(plan, dtype, true, sig, seed, offsets)] = best;
+        g_schedules[schedule_key(plan, dtype, true, sig, seed, offsets)] = Tuned{best, rule_wins};
     }
     if (chosen) *chosen = best;
-    if (best_ms_out) *best_ms_out = best_ms / 2.f;
-    // leave the outputs of the chosen schedule in place
+    if (best_ms_out) *best_ms_out = best_ms;
+    // leave the outputs of what later calls run in place
     return run_signature<T>(plan, s, dtype, incr, offsets, length, batch, sig, sig_stride, seed, seed_stride, grad,
-                            true, best);
+                            true);
 }
 
 // Host buffers in, host buffers out: chunks of the batch go round two
