@@ -16,12 +16,14 @@
 // is what FP32 gains from: the general kernel spends ten instructions a
 // multiply-add and two CTA barriers a degree.  Bound by instruction issue in FP32
 // (0.76 instructions a clock and scheduler at W5 D5), by the pipe in FP64.
-// FP32 sums are formed in short blocks: shorter chains of dependent additions
-// (left W5 D5 78 -> 68 us) and a smaller rounding error.
-// Left / right, general kernel -> this: FP32 W5 D5 batch 4096 112 -> 68 / 119 ->
-// 75 us, W8 D4 111 -> 68 / 117 -> 81, W2 D12 batch 2048 183 -> 111 / 211 -> 152;
-// FP64 W5 D5 221 -> 204 / 233 -> 211, W2 D8 99 -> 47 / 137 -> 73, W2 D12 547 -> 430 /
-// 591 -> 503.
+// FP32 sums are formed in short blocks, these in groups and those in chains: no
+// degree's rounding error is larger than with the terms dealt to the general kernel's
+// 256 threads (rms over both, uniform inputs: 0.6 to 1.06; one chain a lane had 2.1 of
+// it in degree 0 at W5 D5, for 1 % less time).
+// Left / right, general kernel -> this: FP32 W5 D5 batch 4096 111 -> 69 / 117 ->
+// 75 us, W8 D4 110 -> 68 / 117 -> 74, W3 D6 (3000) 51 -> 23 / 52 -> 26, W2 D12 (2048)
+// 183 -> 116 / 211 -> 147; FP64 W5 D5 221 -> 203 / 233 -> 211, W2 D8 99 -> 47 / 136 ->
+// 73, W2 D12 545 -> 429 / 588 -> 498.
 #include <algorithm>
 #include <type_traits>
 
@@ -43,7 +45,7 @@ struct AdjointTasks {
     uint32_t run[kMaxDepth + 1];
 };
 
-AdjointTasks adjoint_tasks(const Geometry& g, bool left, bool fp64, int olo, int ohi, int plo, int phi, int alo, int ahi) {
+AdjointTasks adjoint_tasks(const Geometry& g, bool left, int olo, int ohi, int plo, int phi, int alo, int ahi) {
     AdjointTasks k{};
     uint32_t at = 0;
     for (int m = 0; m <= g.depth; ++m) {
@@ -65,25 +67,96 @@ AdjointTasks adjoint_tasks(const Geometry& g, bool left, bool fp64, int olo, int
     return k;
 }
 
-// acc + sum over i < n, in steps of `step` from `first`, of x[i] y[i ys].  FP32 sums
-// blocks of eight first: a chain of hundreds of additions would double the
-// rounding error of the general kernel's shorter ones.
+// A lane's share of a warp's sum.  FP64: one chain of multiply-adds.  FP32: two
+// chains of blocks of eight terms and two of what is left over -- one chain of the
+// 122 terms that a lane has in degree 0 at W5 D5 has twice the general kernel's
+// rounding error (256 threads of 15 terms), these have the same.
 template <typename T>
-__device__ __forceinline__ T dot(const T* x, const T* y, uint32_t first, uint32_t n, uint32_t step, uint32_t ys, T acc) {
+struct LaneSum {
+    T block0 = T(0), block1 = T(0), rest0 = T(0), rest1 = T(0);
+    __device__ __forceinline__ T total() const {
+        return sizeof(T) == 8 ? block0 : (block0 + block1) + (rest0 + rest1);
+    }
+};
+
+template <typename T>
+__device__ __forceinline__ T eight(const T* x, const T* y, uint32_t i, uint32_t step, uint32_t ys) {
+    T part = x[i] * y[i * ys];
+#pragma unroll
+    for (uint32_t r = 1; r < 8; ++r) part = fma(x[i + r * step], y[(i + r * step) * ys], part);
+    return part;
+}
+
+// Adds x[i] y[i ys], i = first, first + step, ... below n; returns the i after them.
+template <typename T>
+__device__ __forceinline__ uint32_t dot(const T* x, const T* y, uint32_t first, uint32_t n, uint32_t step, uint32_t ys,
+                                        LaneSum<T>& sum) {
+    uint32_t i = first;
     if constexpr (sizeof(T) == 8) {
 #pragma unroll 4
-        for (uint32_t i = first; i < n; i += step) acc = fma(x[i], y[i * ys], acc);
+        for (; i < n; i += step) sum.block0 = fma(x[i], y[i * ys], sum.block0);
     } else {
-        uint32_t i = first;
-        for (; i + 7u * step < n; i += 8u * step) {
-            T part = x[i] * y[i * ys];
-#pragma unroll
-            for (uint32_t r = 1; r < 8; ++r) part = fma(x[i + r * step], y[(i + r * step) * ys], part);
-            acc += part;
+#pragma unroll 1
+        for (; i + 15u * step < n; i += 16u * step) {
+            sum.block0 += eight(x, y, i, step, ys);
+            sum.block1 += eight(x, y, i + 8u * step, step, ys);
         }
-        for (; i < n; i += step) acc = fma(x[i], y[i * ys], acc);
+        if (i + 7u * step < n) {
+            sum.block0 += eight(x, y, i, step, ys);
+            i += 8u * step;
+        }
+#pragma unroll 1
+        for (; i + step < n; i += 2u * step) {
+            sum.rest0 = fma(x[i], y[i * ys], sum.rest0);
+            sum.rest1 = fma(x[i + step], y[(i + step) * ys], sum.rest1);
+        }
+        if (i < n) {
+            sum.rest0 = fma(x[i], y[i * ys], sum.rest0);
+            i += step;
+        }
     }
-    return acc;
+    return i;
+}
+
+// FP32: acc + the terms of split degree p >= 2 (wp = W^p of them) of one coefficient,
+// in blocks of `size` (the multiply-adds that block(part) makes), W blocks to a group,
+// and the groups in a chain: 5 + 5 + 5 additions one after another for the 125 terms
+// of p = 3 at W5.  Two: the blocks of a group in two chains (wide right sums, whose
+// few coefficients had 32 threads each in the general kernel).  Whole: whole groups
+// unrolled (narrow right sums; W3 D6 29.7 -> 26.4 us, but left 22.0 -> 23.1).
+template <int W, bool Two, bool Whole, typename Block>
+__device__ __forceinline__ float grouped(uint32_t wp, float acc, Block&& block) {
+    constexpr uint32_t size = W == 2 ? 4u : W, most = W == 2 ? 4u : W;  // (W = 2: two where p = 3, one where 2)
+    const uint32_t blocks = wp / size < most ? wp / size : most;
+    float sum = 0.0f;
+#pragma unroll 1
+    for (uint32_t i = 0; i < wp; i += blocks * size) {
+        float group = 0.0f;
+        if constexpr (Two) {
+            float other = 0.0f;
+            uint32_t k = 0;
+#pragma unroll 1
+            for (; k + 1 < blocks; k += 2) {
+                group += block(0.0f);
+                other += block(0.0f);
+            }
+            if (k < blocks) group += block(0.0f);
+            group += other;
+        } else {
+            if constexpr (Whole) {
+                if (blocks == most) {
+#pragma unroll
+                    for (uint32_t k = 0; k < most; ++k) group += block(0.0f);
+                    sum += group;
+                    continue;
+                }
+            }
+#pragma unroll(W == 5 ? 1 : 2)
+            for (uint32_t k = 0; k < blocks; ++k) group += block(0.0f);
+        }
+        sum += group;
+    }
+    return acc + sum;
 }
 
 template <typename T, int W, bool Left>
@@ -126,15 +199,16 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
             const int pmin = imax(op.lo, arg.lo - m), pmax = imin(phi, ahi - m);
             T* om = o + G.db[m];
             if (run == 0u) {
-                T acc = T(0);
+                LaneSum<T> sum;
                 if constexpr (Left) {
                     const uint32_t us = 32u / wm, u0 = lane / wm, j = lane - u0 * wm;
                     if (u0 < us)
                         for (int p = pmin; p <= pmax; ++p) {
                             const T* Pp = P + G.db[p];
                             const T* Ap = A + G.db[m + p] + j;
-                            acc = dot(Pp, Ap, u0, G.pw[p], us, wm, acc);
+                            dot(Pp, Ap, u0, G.pw[p], us, wm, sum);
                         }
+                    T acc = sum.total();
                     for (uint32_t off = wm; off < 32u; off *= 2u) {
                         const T x = __shfl_down_sync(0xffffffffu, acc, off);
                         if (lane + off < 32u) acc += x;
@@ -146,10 +220,9 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                         const T* Pp = P + G.db[p];
                         const uint32_t wp = G.pw[p];
                         const T* Ap = A + G.db[m + p] + t * wp;
-#pragma unroll 4
-                        for (; v < wp; v += 32u) acc = fma(Pp[v], Ap[v], acc);
-                        v -= wp;
+                        v = dot(Pp, Ap, v, wp, 32u, 1u, sum) - wp;
                     }
+                    T acc = sum.total();
 #pragma unroll
                     for (uint32_t off = 16u; off > 0u; off /= 2u) acc += __shfl_down_sync(0xffffffffu, acc, off);
                     if (lane == 0) om[t] = acc;
@@ -171,43 +244,67 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                     T v[W];
 #pragma unroll
                     for (int a = 0; a < W; ++a) v[a] = Left ? A1[a * wm + j] : A1[j * W + a];
+                    if constexpr (sizeof(T) == 4 && W >= 5) {  // two shorter chains
+                        T odd = T(0);
 #pragma unroll
-                    for (int a = 0; a < W; ++a) acc = fma(p1[a], v[a], acc);
+                        for (int a = 0; a < W; ++a) (a & 1 ? odd : acc) = fma(p1[a], v[a], a & 1 ? odd : acc);
+                        acc += odd;
+                    } else {
+#pragma unroll
+                        for (int a = 0; a < W; ++a) acc = fma(p1[a], v[a], acc);
+                    }
                 }
                 for (int p = imax(pmin, 2); p <= pmax; ++p) {
                     const T* Pp = P + G.db[p];
                     const uint32_t wp = G.pw[p];
+                    const T* Ap = Left ? A + G.db[m + p] + j : A + G.db[m + p] + j * wp;
+                    constexpr bool two = sizeof(T) == 4 && W >= 7;
                     if constexpr (Left) {
-                        const T* Ap = A + G.db[m + p] + j;
-                        for (uint32_t u = 0; u < wp; u += W, Pp += W, Ap += W * wm) {
-                            T part = sizeof(T) == 4 ? T(0) : acc;  // (FP32: blocks first, as in dot())
+                        auto block = [&](T part) {
+                            constexpr int size = sizeof(T) == 4 && W == 2 ? 4 : W;
 #pragma unroll
-                            for (int a = 0; a < W; ++a) part = fma(Pp[a], Ap[a * wm], part);
-                            acc = sizeof(T) == 4 ? acc + part : part;
-                        }
+                            for (int a = 0; a < size; ++a) part = fma(Pp[a], Ap[a * wm], part);
+                            Pp += size, Ap += size * wm;
+                            return part;
+                        };
+                        if constexpr (sizeof(T) == 4)
+                            acc = grouped<W, false, false>(wp, acc, block);
+                        else
+                            for (uint32_t u = 0; u < wp; u += W) acc = block(acc);
+                    } else if constexpr ((W & (W - 1)) == 0) {
+                        constexpr uint32_t lanes = 128u / sizeof(T);  // of one pass over the banks
+                        uint32_t v = (wp <= lanes ? j * wp / lanes : j) & (wp - 1u);
+                        constexpr uint32_t size = W < 4 ? 4u : W;  // divides wp = W^p, p >= 2
+                        auto block = [&](T part) {
+                            T odd = T(0);
+#pragma unroll
+                            for (uint32_t a = 0; a < size; ++a) {
+                                T& chain = two && (a & 1u) ? odd : part;
+                                chain = fma(Pp[v], Ap[v], chain);
+                                v = (v + 1u) & (wp - 1u);
+                            }
+                            return two ? part + odd : part;
+                        };
+                        if constexpr (sizeof(T) == 4)
+                            acc = grouped<W, two, W <= 4>(wp, acc, block);
+                        else
+                            for (uint32_t i = 0; i < wp; i += size) acc = block(acc);
                     } else {
-                        const T* Ap = A + G.db[m + p] + j * wp;
-                        if constexpr ((W & (W - 1)) == 0) {
-                            constexpr uint32_t lanes = 128u / sizeof(T);  // of one pass over the banks
-                            uint32_t v = (wp <= lanes ? j * wp / lanes : j) & (wp - 1u);
-                            constexpr uint32_t block = W < 4 ? 4u : W;  // divides wp = W^p, p >= 2
-                            for (uint32_t i = 0; i < wp; i += block) {
-                                T part = sizeof(T) == 4 ? T(0) : acc;
+                        uint32_t v = 0;
+                        auto block = [&](T part) {
+                            T odd = T(0);
 #pragma unroll
-                                for (uint32_t a = 0; a < block; ++a) {
-                                    part = fma(Pp[v], Ap[v], part);
-                                    v = (v + 1u) & (wp - 1u);
-                                }
-                                acc = sizeof(T) == 4 ? acc + part : part;
+                            for (int a = 0; a < W; ++a) {
+                                T& chain = two && (a & 1) ? odd : part;
+                                chain = fma(Pp[v + a], Ap[v + a], chain);
                             }
-                        } else {
-                            for (uint32_t v = 0; v < wp; v += W) {
-                                T part = sizeof(T) == 4 ? T(0) : acc;
-#pragma unroll
-                                for (int a = 0; a < W; ++a) part = fma(Pp[v + a], Ap[v + a], part);
-                                acc = sizeof(T) == 4 ? acc + part : part;
-                            }
-                        }
+                            v += W;
+                            return two ? part + odd : part;
+                        };
+                        if constexpr (sizeof(T) == 4)
+                            acc = grouped<W, two, W <= 4>(wp, acc, block);
+                        else
+                            while (v < wp) acc = block(acc);
                     }
                 }
                 om[j] = acc;
@@ -227,7 +324,7 @@ cudaError_t launch_column_adjoint(const Geometry& g, const DeviceInfo& dev, cuda
                                   TArg<T> op, TArg<T> arg, int64_t batch, int64_t arg_group, int staged) {
     const size_t one = static_cast<size_t>(staged_elems<T>(g.dim)) * sizeof(T);
     const size_t smem = kBulkHeader + (staged == 1 ? 2 : staged == 2 ? 1 : 0) * one;
-    const AdjointTasks tasks = adjoint_tasks(g, left, std::is_same<T, double>::value, out.lo, out.hi, op.lo, std::min(op.hi, g.depth), arg.lo,
+    const AdjointTasks tasks = adjoint_tasks(g, left, out.lo, out.hi, op.lo, std::min(op.hi, g.depth), arg.lo,
                                              std::min(arg.hi, g.depth));
     const int threads = g.dim < 256 ? 64 : g.dim < 2048 ? 128 : 256;
     return with_width(g.width, [&](auto w) {
