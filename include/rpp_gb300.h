@@ -455,8 +455,11 @@ int rpp_gb_signature_static_scratch(const rpp_gb_plan* plan, rpp_gb_stream strea
  * rows) -- tried for states whose tensor exceeds 48 KB.  In FP32, bit 16
  * without bit 14 selects the kernels with one warp per first letter and
  * compile-time (width, depth) (forward-only, and forward + reverse for depth
- * >= 3), which FP32 calls of their shapes take when no schedule is recorded.
- * A two-launch winner
+ * >= 3), which FP32 calls of their shapes take when no schedule is recorded --
+ * the forward-only ones of the shapes that rpp_gb_signature_group runs too:
+ * (8, 2..4), (5, 2..5), (4, 4..5), (6, 4), (3, 5..6), (16, 2); of the others,
+ * (2, 2..7), (3, 2..4), (4, 2..3), (4, 6), (6, 2..3), (6, 5), (7, 2..4), no
+ * schedule can ask for them, and *threads never does.  A two-launch winner
  * is refined by timing other reverse sizes, then other forward sizes, and the
  * three fastest schedules with a reverse pass are timed with bit 27 too. */
 int rpp_gb_signature_tune(const rpp_gb_plan* plan, rpp_gb_stream stream, int32_t dtype,
@@ -479,8 +482,9 @@ int rpp_gb_signature_with_schedule(const rpp_gb_plan* plan, rpp_gb_stream stream
  * so one launch covers batches of different (width, depth) and of FP64 and
  * FP32 together, e.g. inside one captured CUDA graph.  Each path of job j is
  * run by a team of `threads` threads (bits 0-9: a multiple of 32, at least
- * width*depth; 0: for FP32 jobs of the shapes of the warp-per-letter kernels
- * (rpp_gb_signature_tune's bit 16) a team of width warps running that code,
+ * width*depth; 0: for FP32 jobs of the shapes whose warp-per-letter kernels
+ * a schedule can ask for (listed at rpp_gb_signature_tune's bit 16) a team of
+ * width warps running that code,
  * otherwise the CTA size of the schedule recorded for that shape by
  * rpp_gb_signature_tune, else a heuristic; bit 26, or a recorded one-launch
  * schedule with bit 26, on an FP64 forward + reverse job: its cotangent level

@@ -284,6 +284,7 @@ struct ScheduleKey {
 };
 struct Tuned {
     int schedule = 0;        // the fastest explicit one (0: never tuned)
+    int team = 0;            // the fastest of the shared-memory kernels', for grouped jobs
     bool rule_wins = false;  // the form chosen by the rule on shape and batch is as fast
 };
 std::mutex g_schedule_lock;
@@ -302,8 +303,10 @@ Tuned tuned(const ScheduleKey& key) {
     return it == g_schedules.end() ? Tuned{} : it->second;
 }
 
-// For the entries that always run an explicit schedule where there is one.
-int scheduled_threads(const ScheduleKey& key) { return tuned(key).schedule; }
+// FP32 schedules of the warp-per-letter kernels.
+bool letter_word(int32_t dtype, int schedule) {
+    return dtype == RPP_GB_F32 && (schedule & rpp_gb::kScheduleLetterWarps) && !(schedule & rpp_gb::kScheduleSplit);
+}
 
 template <typename T>
 int check_signature_args(const rpp_gb_plan* plan, const void* incr, const int64_t* offsets, int64_t length,
@@ -390,10 +393,10 @@ int tune_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const
     // (more CTAs per SM where the whole state holds only one)
     if (sig && !seed)
         for (int t : sizes) candidates[ncand++] = t | rpp_gb::kScheduleForwardTopGlobal;
-    // FP32: the kernels with one warp per first letter (forward-only, and
-    // forward + reverse)
+    // FP32: the kernels with one warp per first letter (forward-only, where a
+    // schedule can ask for them, and forward + reverse)
     if (std::is_same<T, float>::value &&
-        ((sig && !seed && rpp_gb::letter_warps_supported(plan->geometry.width, plan->geometry.depth)) ||
+        ((sig && !seed && rpp_gb::letter_group_supported(plan->geometry.width, plan->geometry.depth)) ||
          (seed && rpp_gb::letter_reverse_supported(plan->geometry.width, plan->geometry.depth))))
         candidates[ncand++] = 32 | rpp_gb::kScheduleLetterWarps;
     // a state split over a cluster of P CTAs by first letter (P divides the
@@ -411,8 +414,8 @@ int tune_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
         return fail(RPP_GB_OUT_OF_RESOURCES, "cudaEventCreate failed");
-    int best = 0;
-    float best_ms = 0.f;
+    int best = 0, team = 0;
+    float best_ms = 0.f, team_ms = 0.f;
     bool device_ok = true;
     // the three fastest candidates so far (ms, schedule), fastest first
     std::pair<float, int> top[3] = {{0.f, 0}, {0.f, 0}, {0.f, 0}};
@@ -443,6 +446,10 @@ int tune_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const
         if (best == 0 || ms < best_ms) {
             best = t;
             best_ms = ms;
+        }
+        if (!letter_word(dtype, t) && (team == 0 || ms < team_ms)) {
+            team = t;
+            team_ms = ms;
         }
         for (int k = 0; k < 3; ++k)
             if (top[k].second == t) return;
@@ -505,7 +512,7 @@ int tune_signature(const rpp_gb_plan* plan, cudaStream_t s, int32_t dtype, const
     if (best == 0) return fail(RPP_GB_NOT_IMPLEMENTED, "no signature schedule can launch for this shape");
     {
         std::lock_guard<std::mutex> guard(g_schedule_lock);
-        g_schedules[schedule_key(plan, dtype, true, sig, seed, offsets)] = Tuned{best, rule_wins};
+        g_schedules[schedule_key(plan, dtype, true, sig, seed, offsets)] = Tuned{best, team, rule_wins};
     }
     if (chosen) *chosen = best;
     if (best_ms_out) *best_ms_out = best_ms;
@@ -1360,7 +1367,13 @@ int rpp_gb_signature_static_scratch(const rpp_gb_plan* plan, rpp_gb_stream strea
                                     int64_t sig_stride, const void* seed, int64_t seed_stride, void* grad) {
     return with_plan(plan, dtype, batch, [&]() -> int {
         auto s = static_cast<cudaStream_t>(stream);
-        const int threads = scheduled_threads(schedule_key(plan, dtype, true, sig, seed, offsets));
+        const Tuned found = tuned(schedule_key(plan, dtype, true, sig, seed, offsets));
+        // (without a schedule this entry runs the same warp-per-letter kernel as
+        // rpp_gb_signature, which a schedule may not be able to ask for)
+        const auto& g = plan->geometry;
+        const bool letters = dtype == RPP_GB_F32 && (seed ? rpp_gb::letter_reverse_supported(g.width, g.depth)
+                                                          : rpp_gb::letter_warps_supported(g.width, g.depth));
+        const int threads = found.rule_wins && letters ? 0 : found.schedule;
         rpp_gb::PathBatch paths{offsets, length, batch};
         rpp_gb::StaticScratchRefusal refusal = rpp_gb::StaticScratchRefusal::None;
         cudaError_t err;
@@ -1436,9 +1449,8 @@ int rpp_gb_signature_group(rpp_gb_stream stream, const rpp_gb_signature_job* job
         if (t == 0) {
             // the recorded schedule's (forward) CTA size and cotangent
             // workspace, else the heuristic
-            int rec = scheduled_threads(schedule_key(job.plan, job.dtype, true, job.sig, job.seed, job.offsets));
-            if (job.dtype == RPP_GB_F32 && (rec & rpp_gb::kScheduleLetterWarps) && !(rec & rpp_gb::kScheduleSplit))
-                rec = 0;  // a warp-per-letter shape that has no team here
+            const Tuned found = tuned(schedule_key(job.plan, job.dtype, true, job.sig, job.seed, job.offsets));
+            const int rec = letter_word(job.dtype, found.schedule) ? found.team : found.schedule;
             t = rec & 1023;
             if (!(rec & rpp_gb::kScheduleSplit) && ((rec >> rpp_gb::kScheduleClusterShift) & 7) == 0)
                 cot = cot || (rec & rpp_gb::kScheduleCotangentGlobal) != 0;
@@ -1486,9 +1498,12 @@ int rpp_gb_signature_with_schedule(const rpp_gb_plan* plan, rpp_gb_stream stream
                                    int32_t schedule) {
     if (schedule <= 0) return fail(RPP_GB_INVALID_ARGUMENT, "schedule must be positive");
     return with_plan(plan, dtype, batch, [&]() -> int {
-        // (the other shapes of the warp-per-letter kernels are taken by the
-        // default and by the autotuner only)
-        if (dtype == RPP_GB_F32 && (schedule & rpp_gb::kScheduleLetterWarps) && !(schedule & rpp_gb::kScheduleSplit) &&
+        // (a forward-only call of the other shapes of the warp-per-letter kernels
+        // takes them without a schedule, which the autotuner times; a word that
+        // asks for them is refused, and never the autotuner's answer)
+        const bool top_in_row = (schedule & rpp_gb::kScheduleForwardTopGlobal) &&
+                                ((schedule >> rpp_gb::kScheduleClusterShift) & 7) == 0;
+        if (letter_word(dtype, schedule) && !seed && !top_in_row &&
             rpp_gb::letter_warps_supported(plan->geometry.width, plan->geometry.depth) &&
             !rpp_gb::letter_group_supported(plan->geometry.width, plan->geometry.depth))
             return cuda_status(cudaErrorInvalidConfiguration, "signature kernel");
