@@ -329,24 +329,71 @@ bool letters_fit(const Geometry& g, const DeviceInfo& dev, int extras) {
     return smem <= std::min(kLettersSmemLimit, static_cast<size_t>(dev.max_smem_optin));
 }
 
-// Where dealing letters is the faster way.  From degree 6 on it has a third of the
-// operations or fewer.  Below, FP32 gains from its plain loops, except where a
-// half-shuffle adjoint of a wide tensor waits at its barriers (W6 D5 left 634 us,
-// 360 by subsets); FP64 only where most of the operations are additions, the
-// products (W4 D4 16.5 -> 13.6; but W8 D4 611, 558 by subsets; left_hs_mul W5 D5
-// 546, 467 by subsets; st_adj_mul W5 D5 1263, 974 by subsets).
+// Where dealing letters is the faster way: from how many tensors an SM on (kAny,
+// kNone).  From degree 6 on it has a third of the operations or fewer.  Below, FP32
+// gains from its plain loops, except where a half-shuffle adjoint of a wide tensor
+// waits at its barriers (W6 D5 left 634 us, 360 by subsets); FP64 only where most of
+// the operations are additions, the products (W4 D4 16.5 -> 13.6; but W8 D4 611, 558
+// by subsets; left_hs_mul W5 D5 546, 467; st_adj_mul W5 D5 1263, 974).
+// The steps are short and end in barriers, which an SM with a CTA or two waits at,
+// where the subset sums have a thread per coefficient and none: six to eight an SM
+// are needed (letters over subsets at batch 64, 608 and 1 300: st_adj_mul FP32 W7 D3
+// 3.1, 1.5 and 1.0; st_mul FP64 W4 D5 2.5, 1.15 and 0.85; left_hs_mul FP64 W2 D7 2.4,
+// 1.45 and 0.85), more for the smallest tensors, two or none where the operations
+// saved outweigh the waits (W3 D6 st_mul FP64 0.9 at batch 64, 0.6 at 4 096).
+// Measured at W 2..8, every depth from 3 to 6 000 coefficients.
+constexpr int kAny = 0, kFew = 2, kSome = 6, kFull = 8, kMany = 20, kNone = 1 << 30;
+
 template <typename T>
-bool letters_pay(const Geometry& g, ShuffleKind kind) {
-    if (std::is_same<T, float>::value || g.depth >= 6) return true;
-    if (kind == ShuffleKind::LeftHalf) return g.dim <= 1200;
-    return g.depth >= 4 && (g.width <= 6 || g.depth >= 5);
+int letters_need(const Geometry& g, ShuffleKind kind) {
+    constexpr bool fp64 = std::is_same<T, double>::value;
+    const int W = g.width, D = g.depth;
+    const bool mid = !fp64 && g.dim >= 1000 && g.dim < 3500;
+    if (kind == ShuffleKind::LeftHalf) {
+        if (fp64 && D < 6 && g.dim > 1200) return kNone;
+        if (D >= (fp64 ? 10 : 9) || (mid && W >= 4) || (D == 3 && (W == 4 || W == 8))) return kAny;
+        if ((W == 2 && D == 5) || (fp64 && D == 4 && W <= 3)) return kNone;
+        if (W == 2 && (D == 4 || D == 6 || (D == 7 && !fp64))) return kMany;
+        if (fp64 && ((W == 3 && D == 5) || (W == 5 && D == 4))) return kMany;
+        if ((W >= 3 && W <= 4 && D >= 6) || (W == 2 && D >= 8 && fp64) || (D == 3 && W >= 6) || (W == 5 && D == 4))
+            return kFew;
+    } else {
+        if (fp64 && (D < 4 || (D == 4 && W > 6))) return kNone;
+        if (D >= (fp64 ? 8 : 9) || (W >= 3 && D >= 6) || mid) return kAny;
+        if (fp64 && D < 6 && W <= 3 && g.dim < 128) return kNone;  // W2 D4, D5, W3 D4
+        if (!fp64 && W <= 3 && g.dim < 128) return kMany;
+        if ((W == 2 && D == 8) || (W >= 5 && g.dim >= 500 && g.dim < 4000)) return kFew;
+    }
+    return g.dim < 256 ? kFull : kSome;
 }
+
 template <typename T>
-bool letters_pay(const Geometry& g, ShuffleAdjKind kind) {
-    if (g.depth >= 6) return true;
-    if (std::is_same<T, double>::value) return false;
-    if (kind == ShuffleAdjKind::HalfL) return g.dim <= 1200;
-    return kind == ShuffleAdjKind::Shuffle || (g.depth >= 4 && g.dim <= 5000);
+int letters_need(const Geometry& g, ShuffleAdjKind kind) {
+    constexpr bool fp64 = std::is_same<T, double>::value;
+    const int W = g.width, D = g.depth;
+    if (fp64 && D < 6) return kNone;
+    if (fp64 && W == 3 && D == 6) return kSome;
+    if (kind == ShuffleAdjKind::Shuffle) {
+        if (W == 2 || D >= 6 || (W == 3 && D <= 4) || (W == 4 && D == 5)) return kAny;
+        // (all first letters at once, in one long pass a degree: 1.3 times the subsets' time)
+        if (W == 7 && D == 4) return kNone;
+        if (D == 4 && (W == 5 || W == 6)) return kFew;
+        return D == 3 && W >= 5 && W <= 7 ? kFull : 4;
+    }
+    if (W >= 4 && D >= 6) return kFew;
+    if (kind == ShuffleAdjKind::HalfL) {
+        if (D < 6 && g.dim > 1200) return kNone;
+        if ((W == 2 && D >= 4) || (W == 3 && (D == 4 || D >= 6))) return kAny;
+        return W == 5 || W == 7 ? kMany : kFull;
+    }
+    if (D < 6 && (D < 4 || g.dim > 5000)) return kNone;
+    if ((W <= 3 && D >= 5) || W == 7) return kAny;
+    return W == 6 || (W == 2 && D == 4) ? kMany : W == 4 ? 4 : kFull;
+}
+
+template <typename T, typename Kind>
+bool letters_pay(const Geometry& g, const DeviceInfo& dev, Kind kind, int64_t batch) {
+    return batch >= static_cast<int64_t>(letters_need<T>(g, kind)) * dev.sm_count;
 }
 
 }  // namespace
@@ -359,7 +406,7 @@ bool shuffle_letters_product_fits(const Geometry& g, const DeviceInfo& dev, Shuf
                                   const TArg<T>& add, const TArg<T>& lhs, const TArg<T>& rhs, int64_t batch) {
     const bool same = add.p == out.p && (batch == 1 || add.stride == out.stride);
     const bool whole = lhs.lo == 0 && rhs.lo == 0 && lhs.hi >= g.depth && rhs.hi >= g.depth;
-    return whole && out.lo <= out.hi && letters_pay<T>(g, kind) && letters_fit<T>(g, dev, kProductExtras) && apart(g, out, lhs, batch) &&
+    return whole && out.lo <= out.hi && letters_pay<T>(g, dev, kind, batch) && letters_fit<T>(g, dev, kProductExtras) && apart(g, out, lhs, batch) &&
            apart(g, out, rhs, batch) && (kind != ShuffleKind::Fma || same || apart(g, out, add, batch));
 }
 
@@ -382,7 +429,7 @@ cudaError_t launch_shuffle_letters_product(const Geometry& g, const DeviceInfo& 
 template <typename T>
 bool shuffle_letters_adjoint_fits(const Geometry& g, const DeviceInfo& dev, ShuffleAdjKind kind, const TArg<T>& out,
                                   const TArg<T>& op, const TArg<T>& arg, int64_t batch) {
-    return out.lo <= out.hi && letters_pay<T>(g, kind) && letters_fit<T>(g, dev, kAdjointExtras) && apart(g, out, op, batch) &&
+    return out.lo <= out.hi && letters_pay<T>(g, dev, kind, batch) && letters_fit<T>(g, dev, kAdjointExtras) && apart(g, out, op, batch) &&
            apart(g, out, arg, batch);
 }
 
