@@ -316,7 +316,30 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
 
 }  // namespace
 
-bool column_adjoint_width(int width) { return column_width(width); }
+// Where it is the faster kernel (the op staged).  Tensors of fewer than 64
+// coefficients are a few warp tasks here, one warp each in the general kernel, which
+// many of them fill the SMs with better (W2 D5 batch 4096: FP64 left 13.7 us, 33.9
+// here; FP32 right 8.7, 14.4; batch 320 FP64 left 0.94 of its time); not for the
+// right adjoint of the smallest FP64 tensors (W4 D3 batch 8192: 24 us, 28 here) and
+// of W4 from depth 5 on (D6, 732: 84, 101); nor for FP64 left W6 D5, whose argument
+// is not staged, where few tensors leave its longest tasks to the end (320: 1.24
+// times the general kernel's).
+template <typename T>
+bool column_adjoint_pays(const Geometry& g, const DeviceInfo& dev, bool left, int staged, int64_t batch) {
+    if (!column_width(g.width)) return false;
+    const int64_t sms = dev.sm_count;
+    const bool wide_flat = g.width >= 6 && g.depth == 2;
+    if (std::is_same<T, double>::value) {
+        if (!left) return g.dim >= 128 && !(g.width == 4 && g.depth >= 5);
+        if (g.dim < 64 && (batch * g.dim >= 184 * sms || g.width == 7 && g.depth == 2)) return false;
+        return !(staged == 2 && g.width == 6 && batch < 4 * sms);
+    }
+    if (g.dim >= 64) return true;
+    if (left) return wide_flat || batch < 13 * sms;
+    return batch < (g.dim >= 30 ? 8 : 13) * sms;
+}
+template bool column_adjoint_pays<float>(const Geometry&, const DeviceInfo&, bool, int, int64_t);
+template bool column_adjoint_pays<double>(const Geometry&, const DeviceInfo&, bool, int, int64_t);
 
 // `staged` as the general launcher chooses it: 0 nothing, 1 both operands, 2 the op.
 template <typename T>

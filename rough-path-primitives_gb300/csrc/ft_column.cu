@@ -110,7 +110,12 @@ size_t column_slot_bytes(const Geometry& g) {
 }  // namespace
 
 template <typename T>
-bool column_product_fits(const Geometry& g, const DeviceInfo& dev) {
+bool column_product_fits(const Geometry& g, const DeviceInfo& dev, bool added, int64_t batch) {
+    // (the general kernel loads the added term before its sum, which few tensors wait for)
+    constexpr Worth kMul32{{60, 125, 300}, {263, 263, 460}, 0, {8, 8, 8}};
+    constexpr Worth kFma32{{150, 500, 700}, {395, 395, 855}, 0, {13, 13, 13}};
+    constexpr Worth kMul64{{100, 100, 2000}, {263, 263, 1974}, 0, {8, 8, 16}};
+    if (!worth(std::is_same<T, double>::value ? kMul64 : added ? kFma32 : kMul32, g, dev, batch)) return false;
     // FP64: where three tensors do not fit shared memory the general kernel
     // runs unstaged, with several CTAs per SM against one here, and is as fast
     // (W6 D5, batch 2048: 283 us against 299); FP32 gains at every size.
@@ -142,7 +147,7 @@ cudaError_t launch_column_product(const Geometry& g, const DeviceInfo& dev, cuda
 }
 
 #define RPP_GB_INSTANTIATE_COLUMN(T)                                                                                 \
-    template bool column_product_fits<T>(const Geometry&, const DeviceInfo&);                                       \
+    template bool column_product_fits<T>(const Geometry&, const DeviceInfo&, bool, int64_t);                                       \
     template cudaError_t launch_column_product<T>(const Geometry&, const DeviceInfo&, cudaStream_t, TArg<T>, TArg<T>, \
                                                 TArg<T>, TArg<T>, int64_t, double, double);
 

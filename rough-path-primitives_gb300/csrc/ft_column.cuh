@@ -242,6 +242,27 @@ inline bool horner_fits(const Geometry& g, const DeviceInfo& dev, size_t smem) {
            smem <= std::min(kHornerSmemLimit, static_cast<size_t>(dev.max_smem_optin));
 }
 
+// Where columns are the faster way.  A thread of them does the work of W to W^2
+// threads of the general kernels one after another, so few tensors, an SM each or
+// less, take longer on columns until a tensor alone has threads' worth of them
+// (`alone` coefficients) or the batch does (`filled` coefficients an SM, of tensors
+// of at least `least`; `many` tensors an SM of any size).  Each field at W = 2, at
+// W = 3 and 4, and at W >= 5, where the columns are W coefficients long.  The lines
+// are where the two kernels' times cross, at W 2..8, every depth to 6 000
+// coefficients and batches of 1 to 4 096 on 152 SMs; on their far side the columns
+// were up to 1.9 times slower (fmexp FP64 W5 D2, 4 096: 7.5 -> 13.8 us), near them
+// either kernel is within 5 %.
+struct Worth {
+    uint32_t alone[3], filled[3], least;
+    uint32_t many[3] = {~0u, ~0u, ~0u};
+};
+constexpr uint32_t kNever = ~0u;
+inline bool worth(const Worth& w, const Geometry& g, const DeviceInfo& dev, int64_t batch) {
+    const int c = g.width == 2 ? 0 : g.width <= 4 ? 1 : 2;
+    if (g.dim >= w.alone[c] || batch >= static_cast<int64_t>(w.many[c]) * dev.sm_count) return true;
+    return g.dim >= w.least && batch * g.dim >= static_cast<int64_t>(w.filled[c]) * dev.sm_count;
+}
+
 // One launch over `groups` CTAs' worth of work, as many at once as fit.
 template <auto kernel, typename... Args>
 inline cudaError_t run_column(const DeviceInfo& dev, cudaStream_t s, int threads, size_t smem, int64_t groups,

@@ -70,7 +70,19 @@ size_t horner_smem(const Geometry& g, bool multiplier) {
 
 template <typename T>
 bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out,
-                        const TArg<T>& x) {
+                        const TArg<T>& x, int64_t batch) {
+    constexpr bool fp64 = std::is_same<T, double>::value;
+    // (depth 1 is one round: columns of exp and fmexp save the others' barriers)
+    constexpr Worth kExp32{{1, 64, 80}, {0, 855, 855}, 0}, kExp64{{100, 64, 700}, {kNever, kNever, 329}, 80};
+    constexpr Worth kLog32{{150, 125, 80}, {658, 658, 329}, 41}, kLog64{{300, 100, 2000}, {6000, 658, 526}, 80};
+    constexpr Worth kFmexp32{{64, 125, 500}, {526, 526, 658}, 41};
+    constexpr Worth kFmexp64{{150, 150, 700}, {329, 200, 1316}, 100};
+    if (!(g.depth == 1 && kind != IntermediateKind::Log) &&
+        !worth(kind == IntermediateKind::Exp ? (fp64 ? kExp64 : kExp32)
+               : kind == IntermediateKind::Log ? (fp64 ? kLog64 : kLog32)
+                                               : (fp64 ? kFmexp64 : kFmexp32),
+               g, dev, batch))
+        return false;
     const bool fm = kind == IntermediateKind::FMExp;
     // (an exponent without degree one leaves degrees of its exponential that have no
     // terms: the general kernel skips them, a product with their zeros would turn
@@ -92,7 +104,7 @@ cudaError_t launch_column_horner(const Geometry& g, const DeviceInfo& dev, cudaS
 
 #define RPP_GB_INSTANTIATE_HORNER(T)                                                                                \
     template bool column_horner_fits<T>(const Geometry&, const DeviceInfo&, IntermediateKind, const TArg<T>&,       \
-                                        const TArg<T>&);                                                        \
+                                        const TArg<T>&, int64_t);                                               \
     template cudaError_t launch_column_horner<T>(const Geometry&, const DeviceInfo&, cudaStream_t, IntermediateKind, \
                                                  TArg<T>, TArg<T>, TArg<T>, int64_t);
 

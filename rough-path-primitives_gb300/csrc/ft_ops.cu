@@ -398,7 +398,8 @@ cudaError_t launch_product(const Geometry& g, const DeviceInfo& dev, cudaStream_
                            TArg<T> out, TArg<T> x, TArg<T> y, TArg<T> z, int64_t batch, double alpha,
                            double beta) {
     if (batch <= 0) return cudaSuccess;
-    if (column_product_fits<T>(g, dev)) {
+    const bool added = kind == ProductKind::Fma ? x.p != nullptr : kind != ProductKind::InplaceMul;
+    if (column_product_fits<T>(g, dev, added, batch)) {
         TArg<T> add{nullptr, 0, 1, 0}, lhs = y, rhs = z;
         switch (kind) {
             case ProductKind::Fma: add = x; break;
@@ -435,7 +436,7 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
     if (kind != IntermediateKind::Log && chen_step_fits<T>(g, dev, out, x))
         return launch_chen_step<T>(g, dev, s, out, kind == IntermediateKind::FMExp ? m : TArg<T>{nullptr, 0, 1, 0}, x,
                                    batch, kind == IntermediateKind::Exp && out.lo == 0);
-    if (column_horner_fits<T>(g, dev, kind, out, x)) return launch_column_horner<T>(g, dev, s, kind, out, x, m, batch);
+    if (column_horner_fits<T>(g, dev, kind, out, x, batch)) return launch_column_horner<T>(g, dev, s, kind, out, x, m, batch);
     constexpr auto kernel = k_intermediate<T>;
     cudaError_t err = allow_large_smem<kernel>(dev);
     if (err != cudaSuccess) return err;
@@ -473,10 +474,7 @@ cudaError_t launch_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_
         staged = 1;
     else if (one + part <= limit)
         staged = 2;
-    // The compile-time-width kernel where the op is staged; not for the right
-    // adjoint of the smallest FP64 tensors (W4 D3 batch 8192: 28 us, 24 here).
-    if (staged && column_adjoint_width(g.width) && out.lo <= out.hi &&
-        !(std::is_same<T, double>::value && !left && g.dim < 128))
+    if (staged && out.lo <= out.hi && column_adjoint_pays<T>(g, dev, left, staged, batch))
         return launch_column_adjoint<T>(g, dev, s, left, out, op, arg, batch, arg_group, staged);
     const size_t smem = (staged == 1 ? 2 * one : staged == 2 ? one : 0) + part;
     const int threads = threads_for(g.pw[g.depth]);

@@ -96,9 +96,13 @@ size_t lie_smem(const Geometry& g, bool multiplier, uint32_t room) {
 }  // namespace
 
 template <typename T>
-bool column_log_to_lie_fits(const Geometry& g, const DeviceInfo& dev, int lo) {
-    // (FP64 at W8, where t2l's rows are most of the time: 250 us, 245 with the general kernel)
-    return lo == 0 && !(std::is_same<T, double>::value && g.width == 8) && horner_fits(g, dev, lie_smem<T>(g, false, lie_room<T>(g, 0)));
+bool column_log_to_lie_fits(const Geometry& g, const DeviceInfo& dev, int lo, int64_t batch) {
+    constexpr Worth k32{{64, 125, 700}, {658, 526, 1118}, 41}, k64{{500, 125, 2000}, {kNever, 1316, 1974}, 0};
+    constexpr bool fp64 = std::is_same<T, double>::value;
+    // (FP64 at W8, and deep tensors of W6 and W7, where t2l's rows are most of the
+    // time: W6 D4 batch 4096 1.23 times the general kernel's, W7 D4 1.12)
+    if (fp64 && (g.width == 8 || (g.width >= 6 && g.dim > 500))) return false;
+    return lo == 0 && worth(fp64 ? k64 : k32, g, dev, batch) && horner_fits(g, dev, lie_smem<T>(g, false, lie_room<T>(g, 0)));
 }
 
 template <typename T>
@@ -116,11 +120,15 @@ cudaError_t launch_column_log_to_lie(const Geometry& g, const DeviceInfo& dev, c
 
 template <typename T>
 bool column_lie_exp_fits(const Geometry& g, const DeviceInfo& dev, const CsrDevice& m, const TArg<T>& out,
-                         bool multiplier, int lo, int hi) {
+                         bool multiplier, int lo, int hi, int64_t batch) {
+    constexpr bool fp64 = std::is_same<T, double>::value;
+    constexpr Worth kExp32{{150, 500, 700}, {526, 855, 1316}, 41}, kExp64{{150, 150, 700}, {0, 0, 1974}, 0};
+    constexpr Worth kFmexp32{{300, 500, 700}, {855, 1500, 1974}, 41}, kFmexp64{{1, 350, 700}, {0, 855, 2400}, 0};
+    if (!worth(multiplier ? (fp64 ? kFmexp64 : kFmexp32) : (fp64 ? kExp64 : kExp32), g, dev, batch)) return false;
     // (an exponent without degree one: see column_horner_fits)
     if (multiplier && (lo > 1 || hi < 1)) return false;
     // (the smallest FP64 tensors, one warp each, gain nothing: W4 D3 37 us, 35 with the general kernel)
-    if (std::is_same<T, double>::value && g.dim < 128) return false;
+    if (fp64 && g.dim < 128) return false;
     return out.lo <= out.hi && (multiplier || out.lo == 0) && m.cols_dim <= static_cast<int64_t>(g.dim) &&
            horner_fits(g, dev, lie_smem<T>(g, multiplier, lie_room<T>(g, m.cols_dim)));
 }
@@ -140,12 +148,12 @@ cudaError_t launch_column_lie_exp(const Geometry& g, const DeviceInfo& dev, cuda
 }
 
 #define RPP_GB_INSTANTIATE_LIE_COLUMN(T)                                                                              \
-    template bool column_log_to_lie_fits<T>(const Geometry&, const DeviceInfo&, int);                               \
+    template bool column_log_to_lie_fits<T>(const Geometry&, const DeviceInfo&, int, int64_t);                               \
     template cudaError_t launch_column_log_to_lie<T>(const Geometry&, const DeviceInfo&, cudaStream_t,              \
                                                      const CsrDevice&, TArg<T>, int, T*, int64_t, int64_t, int64_t, \
                                                      double);                                                       \
     template bool column_lie_exp_fits<T>(const Geometry&, const DeviceInfo&, const CsrDevice&, const TArg<T>&, bool,  \
-                                         int, int);                                                                   \
+                                         int, int, int64_t);                                                                   \
     template cudaError_t launch_column_lie_exp<T>(const Geometry&, const DeviceInfo&, cudaStream_t, const CsrDevice&, \
                                                   const T*, int64_t, int, int, TArg<T>, TArg<T>, int64_t, double);
 

@@ -108,7 +108,7 @@ cudaError_t launch_log_to_lie(const Geometry& g, const DeviceInfo& dev, cudaStre
                               TArg<T> x, int lo, int hi, T* out, int64_t out_stride, int64_t out_size, int64_t batch,
                               double alpha) {
     if (batch <= 0) return cudaSuccess;
-    if (column_log_to_lie_fits<T>(g, dev, lo))
+    if (column_log_to_lie_fits<T>(g, dev, lo, batch))
         return launch_column_log_to_lie<T>(g, dev, s, m, x, hi, out, out_stride, out_size, batch, alpha);
     const size_t smem = log_to_lie_smem(g, sizeof(T));
     if (smem > static_cast<size_t>(dev.max_smem_optin)) return cudaErrorInvalidConfiguration;
@@ -132,7 +132,7 @@ cudaError_t launch_lie_exp(const Geometry& g, const DeviceInfo& dev, cudaStream_
                            const T* lie, int64_t lie_stride, int lo, int hi, TArg<T> out, TArg<T> mult,
                            int64_t batch, double alpha) {
     if (batch <= 0) return cudaSuccess;
-    if (column_lie_exp_fits<T>(g, dev, m, out, mult.p != nullptr, lo, hi))
+    if (column_lie_exp_fits<T>(g, dev, m, out, mult.p != nullptr, lo, hi, batch))
         return launch_column_lie_exp<T>(g, dev, s, m, lie, lie_stride, lo, hi, out, mult, batch, alpha);
     const size_t smem = lie_exp_smem(g, sizeof(T), mult.p != nullptr);
     if (smem > static_cast<size_t>(dev.max_smem_optin) || m.cols_dim > static_cast<int64_t>(g.dim))

@@ -37,7 +37,7 @@ cudaError_t launch_product(const Geometry& g, const DeviceInfo& dev, cudaStream_
 // shared memory) and the one-pass form of exp / fmexp
 // for an exponent of degree one (ft_column.cu).
 template <typename T>
-bool column_product_fits(const Geometry& g, const DeviceInfo& dev);
+bool column_product_fits(const Geometry& g, const DeviceInfo& dev, bool added, int64_t batch);
 template <typename T>
 cudaError_t launch_column_product(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, TArg<T> out, TArg<T> add,
                                 TArg<T> lhs, TArg<T> rhs, int64_t batch, double alpha, double beta);
@@ -50,7 +50,7 @@ cudaError_t launch_chen_step(const Geometry& g, const DeviceInfo& dev, cudaStrea
 // exp / log / fmexp on columns of coefficients (widths 2..8, ft_horner.cu).
 template <typename T>
 bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKind kind, const TArg<T>& out,
-                        const TArg<T>& x);
+                        const TArg<T>& x, int64_t batch);
 template <typename T>
 cudaError_t launch_column_horner(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, IntermediateKind kind,
                                  TArg<T> out, TArg<T> x, TArg<T> m, int64_t batch);
@@ -62,7 +62,8 @@ cudaError_t launch_intermediate(const Geometry& g, const DeviceInfo& dev, cudaSt
 
 // The adjoint multiplies for widths 2..8 (ft_adjoint.cu; `staged` as launch_adjoint
 // chooses it).
-bool column_adjoint_width(int width);
+template <typename T>
+bool column_adjoint_pays(const Geometry& g, const DeviceInfo& dev, bool left, int staged, int64_t batch);
 template <typename T>
 cudaError_t launch_column_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool left, TArg<T> out,
                                   TArg<T> op, TArg<T> arg, int64_t batch, int64_t arg_group, int staged);
@@ -196,14 +197,14 @@ cudaError_t launch_lie_exp(const Geometry& g, const DeviceInfo& dev, cudaStream_
 
 // The same on columns of coefficients (widths 2..8, lie_column.cu).
 template <typename T>
-bool column_log_to_lie_fits(const Geometry& g, const DeviceInfo& dev, int lo);
+bool column_log_to_lie_fits(const Geometry& g, const DeviceInfo& dev, int lo, int64_t batch);
 template <typename T>
 cudaError_t launch_column_log_to_lie(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const CsrDevice& m,
                                      TArg<T> x, int hi, T* out, int64_t out_stride, int64_t out_size, int64_t batch,
                                      double alpha);
 template <typename T>
 bool column_lie_exp_fits(const Geometry& g, const DeviceInfo& dev, const CsrDevice& m, const TArg<T>& out,
-                         bool multiplier, int lo, int hi);
+                         bool multiplier, int lo, int hi, int64_t batch);
 template <typename T>
 cudaError_t launch_column_lie_exp(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, const CsrDevice& m,
                                   const T* lie, int64_t lie_stride, int lo, int hi, TArg<T> out, TArg<T> mult,
