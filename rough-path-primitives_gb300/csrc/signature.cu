@@ -400,11 +400,14 @@ int default_schedule(const SigGeometry& sg, const DeviceInfo& dev, int64_t batch
         return fit(lo + chains) > 0 ? threads(lo + chains) : 0;
     };
     int flags = 0;
+    const size_t fused = dim + lo + 2 * chains;
     if (!forward) {
+        // (an SM with one or two paths has room for their top levels, and waits for
+        // every read of a row: W6 D5, 8 paths x 64 1 210 us from the row, 895 on chip)
+        if (want <= 2 && fit(fused) >= want) return threads(fused) | merged;
         const int t = reverse_part(flags);
         return t > 0 ? t | flags | kScheduleForwardTopGlobal : 0;
     }
-    const size_t fused = dim + lo + 2 * chains;
     if (fit(fused) >= want || (!has_sig && fit(fused) >= 4)) return threads(fused) | merged;
     if (!has_sig) return fit(dim + chains) > 0 ? threads(dim + chains) | kScheduleCotangentGlobal : 0;
     if (split_state) return in_cluster | kScheduleCotangentGlobal;
