@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
     __shared__ uint32_t s_next;
     const uint32_t pd = staged_elems<T>(G.dim);
     uint32_t phase = 0;
-    if (staged) bulk_stage_init(bar);
+    bulk_stage_init(bar);
     const int D = G.depth;
     const int ohi = imin(out.hi, D), phi = imin(op.hi, D), ahi = imin(arg.hi, D);
     const uint32_t lane = threadIdx.x & 31u;
@@ -178,14 +178,10 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
         const T* A = arg.at(arg_group == 1 ? b : b / arg_group);
         T* o = out.at(b);
         if (threadIdx.x == 0) s_next = 0;
-        if (staged) {
-            BulkStage<T> st(bar, phase);
-            P = st.add(sm, P, op.lo, phi, G);
-            if (staged == 1) A = st.add(sm + pd, A, arg.lo, ahi, G);
-            if (!st.commit(G.fault)) return;
-        } else {
-            __syncthreads();
-        }
+        BulkStage<T> st(bar, phase);
+        P = st.add(sm, P, op.lo, phi, G);
+        if (staged == 1) A = st.add(sm + pd, A, arg.lo, ahi, G);
+        if (!st.commit(G.fault)) return;
         for (;;) {
             uint32_t t = 0;
             if (lane == 0) t = atomicAdd(&s_next, 1u);
@@ -341,12 +337,12 @@ bool column_adjoint_pays(const Geometry& g, const DeviceInfo& dev, bool left, in
 template bool column_adjoint_pays<float>(const Geometry&, const DeviceInfo&, bool, int, int64_t);
 template bool column_adjoint_pays<double>(const Geometry&, const DeviceInfo&, bool, int, int64_t);
 
-// `staged` as the general launcher chooses it: 0 nothing, 1 both operands, 2 the op.
+// `staged` as the general launcher chooses it: 1 both operands, 2 the op.
 template <typename T>
 cudaError_t launch_column_adjoint(const Geometry& g, const DeviceInfo& dev, cudaStream_t s, bool left, TArg<T> out,
                                   TArg<T> op, TArg<T> arg, int64_t batch, int64_t arg_group, int staged) {
     const size_t one = static_cast<size_t>(staged_elems<T>(g.dim)) * sizeof(T);
-    const size_t smem = kBulkHeader + (staged == 1 ? 2 : staged == 2 ? 1 : 0) * one;
+    const size_t smem = kBulkHeader + (staged == 1 ? 2 : 1) * one;
     const AdjointTasks tasks = adjoint_tasks(g, left, out.lo, out.hi, op.lo, std::min(op.hi, g.depth), arg.lo,
                                              std::min(arg.hi, g.depth));
     const int threads = g.dim < 256 ? 64 : g.dim < 2048 ? 128 : 256;

@@ -386,11 +386,7 @@ constexpr size_t kStageLimit = 200 * 1024;
 // written: it lies apart from the output, or is the output itself.
 template <typename T>
 static bool add_in_place(const Geometry& g, const TArg<T>& out, const TArg<T>& add, int64_t batch) {
-    if (!add.p || add.lo > add.hi || out.lo > out.hi) return true;
-    if (add.p == out.p && (batch == 1 || add.stride == out.stride)) return true;
-    auto begin = [&](const TArg<T>& t) { return t.p + g.db[t.lo]; };
-    auto end = [&](const TArg<T>& t) { return t.p + (batch - 1) * t.stride + g.db[std::min(t.hi, g.depth) + 1]; };
-    return end(add) <= begin(out) || end(out) <= begin(add);
+    return (add.p == out.p && (batch == 1 || add.stride == out.stride)) || apart(g, out, add, batch);
 }
 
 template <typename T>

@@ -68,6 +68,15 @@ inline cudaError_t batch_grid(Kernel kernel, const DeviceInfo& dev, int threads,
     return cudaSuccess;
 }
 
+// Whether two operand batches share no memory (empty ones share none).
+template <typename T>
+inline bool apart(const Geometry& g, const TArg<T>& a, const TArg<T>& b, int64_t batch) {
+    if (!a.p || !b.p || a.lo > a.hi || b.lo > b.hi) return true;
+    auto begin = [&](const TArg<T>& t) { return t.p + g.db[t.lo]; };
+    auto end = [&](const TArg<T>& t) { return t.p + (batch - 1) * t.stride + g.db[std::min(t.hi, g.depth) + 1]; };
+    return end(a) <= begin(b) || end(b) <= begin(a);
+}
+
 // Threads per CTA for a tensor whose largest level has `widest` coefficients.
 inline int threads_for(uint32_t widest, int cap = 256) {
     int t = 32;

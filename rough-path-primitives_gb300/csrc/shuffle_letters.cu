@@ -293,14 +293,6 @@ __global__ void __launch_bounds__(512) k_deal_product(Geometry G, PowerDiv pd, i
     }
 }
 
-template <typename T>
-bool apart(const Geometry& g, const TArg<T>& a, const TArg<T>& b, int64_t batch) {
-    if (!a.p || !b.p || a.lo > a.hi || b.lo > b.hi) return true;
-    auto begin = [&](const TArg<T>& t) { return t.p + g.db[t.lo]; };
-    auto end = [&](const TArg<T>& t) { return t.p + (batch - 1) * t.stride + g.db[std::min(t.hi, g.depth) + 1]; };
-    return end(a) <= begin(b) || end(b) <= begin(a);
-}
-
 // First letters at a time, shared memory and threads (four words each) of a
 // launch: all first letters where six CTAs still fit an SM, else one.
 template <typename T>
@@ -342,7 +334,7 @@ bool letters_fit(const Geometry& g, const DeviceInfo& dev, int extras) {
 // 1.45 and 0.85), more for the smallest tensors, two or none where the operations
 // saved outweigh the waits (W3 D6 st_mul FP64 0.9 at batch 64, 0.6 at 4 096).
 // Measured at W 2..8, every depth from 3 to 6 000 coefficients.
-constexpr int kAny = 0, kFew = 2, kSome = 6, kFull = 8, kMany = 20, kNone = 1 << 30;
+enum : int { kAny = 0, kFew = 2, kSome = 6, kFull = 8, kMany = 20, kNone = 1 << 30 };
 
 template <typename T>
 int letters_need(const Geometry& g, ShuffleKind kind) {

@@ -32,15 +32,14 @@ constexpr size_t kJoinSmemLimit = 200 * 1024;
 // operands too large for shared memory (read in place, top level first).
 template <typename T, int WT>
 __device__ void join(const Geometry& G, T* out, T* also, const T* L, const T* R, uint64_t* bar, uint32_t& phase,
-                     T* sm, bool& ok) {
+                     T* sm) {
     const int D = G.depth;
     if constexpr (WT > 0) {
         const uint32_t pd = staged_elems<T>(G.dim);
         BulkStage<T> st(bar, phase);
         const T* l = st.add(sm, L, 0, D, G);
         const T* r = st.add(sm + pd, R, 0, D, G);
-        ok = st.commit(G.fault);
-        if (!ok) return;
+        if (!st.commit(G.fault)) return;
         const uint32_t tasks = tensor_tasks<T, WT>(G, 0, D);
         for (uint32_t t = threadIdx.x; t < tasks; t += blockDim.x) {
             int n;
@@ -76,14 +75,13 @@ __global__ void __launch_bounds__(kJoinThreads) k_chunk_reduce(Geometry G, T* pi
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
     uint32_t phase = 0;
-    bool ok = true;
     if (WT > 0) bulk_stage_init(bar);
     const int64_t path = blockIdx.x / pairs, c = (blockIdx.x - path * pairs) << (r + 1);
     T* l = pieces + (path * chunks + c) * pitch;
     const T* rr = l + (static_cast<int64_t>(1) << r) * pitch;
     const bool last = (static_cast<int64_t>(2) << r) >= chunks;
     join<T, WT>(G, last ? sig + path * sig_stride : l, nullptr, l, rr, bar, phase,
-                reinterpret_cast<T*>(smem_raw + kBulkHeader), ok);
+                reinterpret_cast<T*>(smem_raw + kBulkHeader));
 }
 
 // Round `r` of both scans (Sklansky's: a piece whose index has bit r set takes
@@ -96,7 +94,6 @@ __global__ void __launch_bounds__(kJoinThreads) k_chunk_scan(Geometry G, const T
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
     uint32_t phase = 0;
-    bool ok = true;
     const int64_t path = blockIdx.x / chunks, c = blockIdx.x - path * chunks;
     const bool suffix = blockIdx.y != 0;
     const int64_t i = suffix ? chunks - 1 - c : c;  // index in the direction of the scan
@@ -121,7 +118,7 @@ __global__ void __launch_bounds__(kJoinThreads) k_chunk_scan(Geometry G, const T
     }
     if (WT > 0) bulk_stage_init(bar);
     join<T, WT>(G, own, also, suffix ? mine : other, suffix ? other : mine, bar, phase,
-                reinterpret_cast<T*>(smem_raw + kBulkHeader), ok);
+                reinterpret_cast<T*>(smem_raw + kBulkHeader));
 }
 
 template <typename T>
