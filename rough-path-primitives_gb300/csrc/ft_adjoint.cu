@@ -16,14 +16,16 @@
 // is what FP32 gains from: the general kernel spends ten instructions a
 // multiply-add and two CTA barriers a degree.  Bound by instruction issue in FP32
 // (0.76 instructions a clock and scheduler at W5 D5), by the pipe in FP64.
-// FP32 sums are formed in short blocks, these in groups and those in chains: no
-// degree's rounding error is larger than with the terms dealt to the general kernel's
-// 256 threads (rms over both, uniform inputs: 0.6 to 1.06; one chain a lane had 2.1 of
-// it in degree 0 at W5 D5, for 1 % less time).
-// Left / right, general kernel -> this: FP32 W5 D5 batch 4096 111 -> 69 / 117 ->
-// 75 us, W8 D4 110 -> 68 / 117 -> 74, W3 D6 (3000) 51 -> 23 / 52 -> 26, W2 D12 (2048)
-// 183 -> 116 / 211 -> 147; FP64 W5 D5 221 -> 203 / 233 -> 211, W2 D8 99 -> 47 / 136 ->
-// 73, W2 D12 545 -> 429 / 588 -> 498.
+// FP32 sums are formed in short blocks, these in groups and those in chains; FP64
+// sums of 12 terms or more have two to eight chains where the general kernel has as
+// many threads for a coefficient.  Neither rounds more than its 256 threads a tensor
+// do (rms error over both, uniform inputs: FP32 0.6 to 1.06, FP64 0.7 to 1.2 in a
+// degree and 1.0 in most; one chain a lane had up to 2.8 times that, W6 D5 degree 0).
+// Left / right, general kernel -> this: FP32 W5 D5 batch 4096 111 -> 65 / 117 ->
+// 67 us, W8 D4 110 -> 65 / 117 -> 71, W3 D6 (3000) 51 -> 22 / 52 -> 23, W2 D12 (2048)
+// 183 -> 109 / 211 -> 137; FP64 W5 D5 221 -> 209 / 233 -> 224, W2 D8 99 -> 48 / 136 ->
+// 75, W2 D12 545 -> 426 / 588 -> 518 (with one chain a lane 203 / 211, 47 / 73 and
+// 429 / 497).
 #include <algorithm>
 #include <type_traits>
 
@@ -67,15 +69,21 @@ AdjointTasks adjoint_tasks(const Geometry& g, bool left, int olo, int ohi, int p
     return k;
 }
 
-// A lane's share of a warp's sum.  FP64: one chain of multiply-adds.  FP32: two
-// chains of blocks of eight terms and two of what is left over -- one chain of the
-// 122 terms that a lane has in degree 0 at W5 D5 has twice the general kernel's
-// rounding error (256 threads of 15 terms), these have the same.
+// A lane's share of a warp's sum.  One chain of the 122 terms that a lane has in
+// degree 0 at W5 D5 has twice the general kernel's rounding error (256 threads of 15
+// terms), these have the same.  FP32: two chains of blocks of eight terms and two of
+// what is left over.  FP64, whose additions are dear: eight chains (`wide`: where a
+// lane has 16 terms or more), or one.
 template <typename T>
 struct LaneSum {
     T block0 = T(0), block1 = T(0), rest0 = T(0), rest1 = T(0);
-    __device__ __forceinline__ T total() const {
-        return sizeof(T) == 8 ? block0 : (block0 + block1) + (rest0 + rest1);
+    __device__ __forceinline__ T total(bool) const { return (block0 + block1) + (rest0 + rest1); }
+};
+template <>
+struct LaneSum<double> {
+    double r[8] = {};
+    __device__ __forceinline__ double total(bool wide) const {
+        return wide ? ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7])) : r[0];
     }
 };
 
@@ -90,11 +98,15 @@ __device__ __forceinline__ T eight(const T* x, const T* y, uint32_t i, uint32_t 
 // Adds x[i] y[i ys], i = first, first + step, ... below n; returns the i after them.
 template <typename T>
 __device__ __forceinline__ uint32_t dot(const T* x, const T* y, uint32_t first, uint32_t n, uint32_t step, uint32_t ys,
-                                        LaneSum<T>& sum) {
+                                        LaneSum<T>& sum, bool wide) {
     uint32_t i = first;
     if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+        for (; wide && i + 7u * step < n; i += 8u * step)
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q) sum.r[q] = fma(x[i + q * step], y[(i + q * step) * ys], sum.r[q]);
 #pragma unroll 4
-        for (; i < n; i += step) sum.block0 = fma(x[i], y[i * ys], sum.block0);
+        for (; i < n; i += step) sum.r[0] = fma(x[i], y[i * ys], sum.r[0]);
     } else {
 #pragma unroll 1
         for (; i + 15u * step < n; i += 16u * step) {
@@ -159,6 +171,46 @@ __device__ __forceinline__ float grouped(uint32_t wp, float acc, Block&& block) 
     return acc + sum;
 }
 
+// FP64: the terms of split degrees plo..phi (plo >= 2) of coefficient j of degree m in
+// `chains` chains (2, 4 or 8), the blocks of W terms taken in turn.
+template <typename T, int W, bool Left>
+__device__ __forceinline__ T spread_sum(const Geometry& G, const T* P, const T* A, int m, uint32_t j, int plo, int phi,
+                                        uint32_t wm, uint32_t chains) {
+    constexpr uint32_t size = W == 2 ? 4u : W;  // divides W^p, p >= 2
+    constexpr bool rotate = !Left && (W & (W - 1)) == 0;
+    constexpr uint32_t lanes = 128u / sizeof(T);  // of one pass over the banks
+    T r[8] = {};
+    for (int p = plo; p <= phi; ++p) {
+        const uint32_t wp = G.pw[p];
+        const T* Pp = P + G.db[p];
+        const T* Ap = A + G.db[m + p] + (Left ? j : j * wp);
+        uint32_t v = rotate ? (wp <= lanes ? j * wp / lanes : j) & (wp - 1u) : 0u;
+        auto block = [&](auto&& put) {
+#pragma unroll
+            for (uint32_t a = 0; a < size; ++a) {
+                put(a, Pp[v], Ap[Left ? v * wm : v]);
+                v = rotate ? (v + 1u) & (wp - 1u) : v + 1u;
+            }
+        };
+        const uint32_t blocks = wp / size;
+        if (chains == 2u) {
+            for (uint32_t k = 0; k < blocks; ++k) block([&](uint32_t a, T x, T y) { r[a & 1u] = fma(x, y, r[a & 1u]); });
+        } else if (chains == 4u) {
+            for (uint32_t k = 0; k < blocks; ++k) block([&](uint32_t a, T x, T y) { r[a & 3u] = fma(x, y, r[a & 3u]); });
+        } else {
+            uint32_t k = 0;
+            for (; k + 1u < blocks; k += 2u) {
+                block([&](uint32_t a, T x, T y) { r[a & 3u] = fma(x, y, r[a & 3u]); });
+                block([&](uint32_t a, T x, T y) { r[4u + (a & 3u)] = fma(x, y, r[4u + (a & 3u)]); });
+            }
+            if (k < blocks) block([&](uint32_t a, T x, T y) { r[a & 3u] = fma(x, y, r[a & 3u]); });
+        }
+    }
+    if (chains == 2u) return r[0] + r[1];
+    if (chains == 4u) return (r[0] + r[1]) + (r[2] + r[3]);
+    return ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
+}
+
 template <typename T, int W, bool Left>
 __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out, TArg<T> op, TArg<T> arg,
                                                         int64_t batch, int64_t arg_group, int staged,
@@ -196,15 +248,17 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
             T* om = o + G.db[m];
             if (run == 0u) {
                 LaneSum<T> sum;
+                const bool wide = sizeof(T) == 8 && pmin <= pmax &&
+                                  G.db[pmax + 1] - G.db[pmin] >= 16u * (Left ? 32u / wm : 32u);
                 if constexpr (Left) {
                     const uint32_t us = 32u / wm, u0 = lane / wm, j = lane - u0 * wm;
                     if (u0 < us)
                         for (int p = pmin; p <= pmax; ++p) {
                             const T* Pp = P + G.db[p];
                             const T* Ap = A + G.db[m + p] + j;
-                            dot(Pp, Ap, u0, G.pw[p], us, wm, sum);
+                            dot(Pp, Ap, u0, G.pw[p], us, wm, sum, wide);
                         }
-                    T acc = sum.total();
+                    T acc = sum.total(wide);
                     for (uint32_t off = wm; off < 32u; off *= 2u) {
                         const T x = __shfl_down_sync(0xffffffffu, acc, off);
                         if (lane + off < 32u) acc += x;
@@ -216,9 +270,9 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                         const T* Pp = P + G.db[p];
                         const uint32_t wp = G.pw[p];
                         const T* Ap = A + G.db[m + p] + t * wp;
-                        v = dot(Pp, Ap, v, wp, 32u, 1u, sum) - wp;
+                        v = dot(Pp, Ap, v, wp, 32u, 1u, sum, wide) - wp;
                     }
-                    T acc = sum.total();
+                    T acc = sum.total(wide);
 #pragma unroll
                     for (uint32_t off = 16u; off > 0u; off /= 2u) acc += __shfl_down_sync(0xffffffffu, acc, off);
                     if (lane == 0) om[t] = acc;
@@ -226,6 +280,11 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                 continue;
             }
             const uint32_t last = (t + 1u) * run, end = last < wm ? last : wm;
+            // FP64: where the general kernel has several threads for a coefficient of many
+            // terms, its sum has several chains here
+            const uint32_t terms = pmin <= pmax ? G.db[pmax + 1] - G.db[pmin] : 0u;
+            const bool spread = sizeof(T) == 8 && wm < 200u && terms >= 12u;
+            const uint32_t chains = wm >= 100u || terms < 24u ? 2u : terms < 64u ? 4u : 8u;
             const bool has0 = pmin <= 0 && pmax >= 0, has1 = pmin <= 1 && pmax >= 1;
             const T p0 = has0 ? P[0] : T(0);
             T p1[W];
@@ -240,7 +299,7 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                     T v[W];
 #pragma unroll
                     for (int a = 0; a < W; ++a) v[a] = Left ? A1[a * wm + j] : A1[j * W + a];
-                    if constexpr (sizeof(T) == 4 && W >= 5) {  // two shorter chains
+                    if (W >= 5 && (sizeof(T) == 4 || spread)) {  // two shorter chains
                         T odd = T(0);
 #pragma unroll
                         for (int a = 0; a < W; ++a) (a & 1 ? odd : acc) = fma(p1[a], v[a], a & 1 ? odd : acc);
@@ -248,6 +307,12 @@ __global__ void __launch_bounds__(256) k_column_adjoint(Geometry G, TArg<T> out,
                     } else {
 #pragma unroll
                         for (int a = 0; a < W; ++a) acc = fma(p1[a], v[a], acc);
+                    }
+                }
+                if constexpr (sizeof(T) == 8) {
+                    if (spread) {
+                        om[j] = acc + spread_sum<T, W, Left>(G, P, A, m, j, imax(pmin, 2), pmax, wm, chains);
+                        continue;
                     }
                 }
                 for (int p = imax(pmin, 2); p <= pmax; ++p) {

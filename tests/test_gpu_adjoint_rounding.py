@@ -1,4 +1,4 @@
-"""Rounding of the FP32 adjoint multiplies (csrc/ft_adjoint.cu): per degree, no
+"""Rounding of the adjoint multiplies (csrc/ft_adjoint.cu): per degree, no
 more than a coefficient's terms dealt to the 256 threads of the general kernel
 (csrc/ft_ops.cu) and summed pairwise, on the same inputs."""
 import importlib
@@ -67,3 +67,49 @@ def test_fp32_sums_round_no_more_than_the_dealt_ones(W, D, left):
         # of the ratio of two measured values are 13 %
         ours, theirs = rms(got[:few, db[m]:db[m + 1]]), rms(dealt(x, y, W, D, m))
         assert ours <= 1.25 * theirs, (m, ours, theirs)
+
+
+def dealt_fp64(x, y, W, D, m):
+    """dealt() in FP64: each multiply-add formed in the wider type and rounded once."""
+    nt, threads = 32, 1
+    while nt < 256 and nt < W ** D:
+        nt *= 2
+    while 2 * threads * W ** m <= nt:
+        threads *= 2
+    sums = []
+    for r in range(threads):
+        acc = np.zeros(y.shape[:2])
+        for k in range(r, y.shape[2], threads):
+            acc = (x[..., k].astype(np.longdouble) * y[..., k] + acc).astype(np.float64)
+        sums.append(acc)
+    while len(sums) > 1:
+        sums = [a + b for a, b in zip(sums[::2], sums[1::2])]
+    return sums[0]
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).nmant < 106, reason="needs products of FP64 numbers exactly")
+@pytest.mark.parametrize("W,D", [(2, 5), (2, 8), (3, 5), (4, 5), (5, 4), (5, 5), (6, 4), (7, 3), (8, 3)])
+@pytest.mark.parametrize("left", [True, False])
+def test_fp64_sums_round_no_more_than_the_dealt_ones(W, D, left):
+    rng = np.random.default_rng(W * 10 + D)
+    db = starts(W, D)
+    B = 1000
+    op, arg = (rng.uniform(-1, 1, (B, db[-1])) for _ in range(2))
+    basis, st = pkg.TensorBasis(W, D), pkg.GB300Strategy(torch.float64)
+    out = torch.empty(B, int(db[-1]), dtype=torch.float64, device="cuda")
+    batch = lambda t: pkg.make_tensor_batch(t, basis.size(), 0, D)  # noqa: E731
+    multiply = pkg.ft_adj_lmul if left else pkg.ft_adj_rmul
+    assert multiply(st, None, batch(out), *(batch(torch.from_numpy(v).cuda()) for v in (op, arg)), basis, B)
+    got = out.cpu().numpy()
+    for m in range(D + 1):
+        few = max(8, min(B, 100_000 // int(db[-1])), 1000 // W ** m)
+        x, y = terms(op[:few], arg[:few], W, D, m, left)
+        want = (x.astype(np.longdouble) * y).sum(-1)
+
+        def rms(v):
+            return float(np.sqrt(((v.astype(np.longdouble) - want) ** 2).mean()))
+
+        # (the orders differ by up to 18 % by design, where a lane sums what 16 threads
+        # or more did; four deviations of the ratio of two measured values are 13 %)
+        ours, theirs = rms(got[:few, db[m]:db[m + 1]]), rms(dealt_fp64(x, y, W, D, m))
+        assert ours <= 1.33 * theirs, (m, ours, theirs)
