@@ -205,19 +205,47 @@ __device__ __forceinline__ void horner_in_place(const Geometry& G, int H, T* x, 
     __syncthreads();
 }
 
-// out = M (x) E on out's degrees, E at `e` to degree he, M staged at `m` (levels
-// mlo..mhi).
+// o's degrees [olo, ohi] = M (x) exp(X), M (levels mlo >= olo .. mhi) and X (xlo >= 1
+// .. xhi) staged, by Horner's rule on the multiplier: p_d = M + p_{d+1} (x) X / d, d =
+// ohi - mlo .. 1.  X has no degree 0, so round d forms the levels up to ohi - d + 1
+// only, the ones that later rounds read, as exp's rounds do: 22 k multiply-adds at W5
+// D5, where exp and one product take 41 k and carry the rounding of exp's coefficients
+// into the result.  The last and largest round divides by 1, so exp's rescaling, which
+// would round M itself, saves nothing here.  The running tensor alternates between two
+// buffers of the levels below ohi, one barrier a round.
 template <typename T, int W>
-__device__ __forceinline__ void multiply_out(const Geometry& G, T* o, int olo, int ohi, const T* m, int mlo, int mhi,
-                                             const T* e, int he) {
-    const uint32_t tasks = tensor_tasks<T, W>(G, olo, ohi);
-    for (uint32_t t = threadIdx.x; t < tasks; t += blockDim.x) {
-        int n;
-        uint32_t i, place;
-        locate_task<T, W>(G, t, 1, ohi, n, i, place);
-        T* dst = o + G.db[n];
-        task_product<T, W>(G, Opnd<T>{m, mlo, mhi}, Opnd<T>{e, 0, he}, n, place,
-                           [&](uint32_t at, T v) { dst[at] = v; });
+__device__ __forceinline__ void horner_multiplied(const Geometry& G, T* o, int olo, int ohi, const T* m, int mlo,
+                                                  int mhi, const Opnd<T>& X, T* cur, T* next) {
+    const auto& rc = ftdev::recip<T>();
+    const bool empty = mlo > mhi || mlo > ohi;
+    const uint32_t below = G.db[empty ? ohi + 1 : mlo];
+    for (uint32_t i = G.db[olo] + threadIdx.x; i < below; i += blockDim.x) o[i] = T(0);
+    if (empty) return;
+    const int H = ohi - mlo;
+    T* start = H > 0 ? cur : o;  // (no exponent reaches the multiplier's only level)
+    for (uint32_t i = G.db[mlo] + threadIdx.x; i < G.db[mlo + 1]; i += blockDim.x) start[i] = m[i];
+    __syncthreads();
+    for (int d = H; d > 0; --d) {
+        const int t = ohi - d + 1;
+        const uint32_t tasks = tensor_tasks<T, W>(G, mlo, t);
+        const Opnd<T> L{cur, mlo, t - 1}, R{X.p, X.lo, imin(X.hi, t - mlo)};
+        const T inv = rc.inv[d];
+        T* to = d > 1 ? next : o;
+        for (uint32_t i = threadIdx.x; i < tasks; i += blockDim.x) {
+            int n;
+            uint32_t tensor, place;
+            locate_task<T, W>(G, i, 1, t, n, tensor, place);
+            const T* mn = n <= mhi ? m + G.db[n] : nullptr;
+            T* row = to + G.db[n];
+            task_product<T, W>(G, L, R, n, place, [&](uint32_t at, T v) {
+                if (d > 1) row[at] = mn ? fma(v, inv, mn[at]) : v * inv;
+                else row[at] = mn ? v + mn[at] : v;
+            });
+        }
+        __syncthreads();
+        T* swap = cur;
+        cur = next;
+        next = swap;
     }
 }
 
@@ -250,7 +278,7 @@ inline bool horner_fits(const Geometry& g, const DeviceInfo& dev, size_t smem) {
 // W = 3 and 4, and at W >= 5, where the columns are W coefficients long.  The lines
 // are where the two kernels' times cross, at W 2..8, every depth to 6 000
 // coefficients and batches of 1 to 4 096 on 152 SMs; on their far side the columns
-// were up to 1.9 times slower (fmexp FP64 W5 D2, 4 096: 7.5 -> 13.8 us), near them
+// were up to 2.5 times slower (left adjoint FP64 W2 D5, 4 096: 13.7 -> 33.9 us), near them
 // either kernel is within 5 %.
 struct Worth {
     uint32_t alone[3], filled[3], least;

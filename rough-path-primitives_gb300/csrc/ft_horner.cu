@@ -1,7 +1,6 @@
 // ft_horner.cu -- ft_exp, ft_log and ft_fmexp for widths 2..8: Horner's rule on
 // columns of coefficients (ft_column.cuh), each round only on the levels that
-// later rounds read.  fmexp is exp and then one product, 41 k multiply-adds at
-// W5 D5, where Horner's rule on the multiplier takes 57 k.
+// later rounds read; fmexp is Horner's rule on the multiplier.
 #include <algorithm>
 #include <type_traits>
 
@@ -18,9 +17,10 @@ using namespace ftcol;
 
 // ft_exp, ft_log (out from degree 0) and ft_fmexp.  FP64 is bound by its pipe,
 // FP32 by the rounds' latency.  Batch 4096, general kernel -> this: exp W5 D5
-// FP64 511 -> 200 us, FP32 311 -> 69; log FP64 212 -> 191, FP32 127 -> 69; fmexp
-// FP64 718 -> 404, FP32 355 -> 108; W2 D12 (2 048) exp FP64 3249 -> 983, FP32
-// 1242 -> 193.
+// FP64 511 -> 200 us, FP32 311 -> 64; log FP64 212 -> 191, FP32 127 -> 69; fmexp
+// FP64 717 -> 273, FP32 354 -> 75 (405 and 107 as exp and one product, whose rounding
+// error is also 1.3 to 1.8 times as large); W2 D12 (2 048) exp FP64 3247 -> 983, FP32
+// 1243 -> 176, fmexp 3607 -> 1021 and 1473 -> 239.
 template <typename T, int W>
 __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_column_horner(Geometry G, IntermediateKind kind, TArg<T> out,
                                                                   TArg<T> x, TArg<T> m, int64_t batch) {
@@ -45,8 +45,7 @@ __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_colum
         if (!st.commit(G.fault)) return;
         T* o = out.at(b);
         if (fm) {
-            horner_in_place<T, W, false>(G, H, X, xlo, xhi, buf, half);
-            multiply_out<T, W>(G, o, out.lo, ohi, M, mlo, mhi, X, H);
+            horner_multiplied<T, W>(G, o, out.lo, ohi, M, mlo, mhi, Opnd<T>{X, xlo, xhi}, buf, buf + half);
         } else if (kind == IntermediateKind::Exp) {
             const T unit = horner<T, W, false>(G, H, Opnd<T>{X, xlo, xhi}, buf, buf + half,
                                                [&](int n, uint32_t at, T v) { o[G.db[n] + at] = v; });
@@ -75,8 +74,7 @@ bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKi
     // (depth 1 is one round: columns of exp and fmexp save the others' barriers)
     constexpr Worth kExp32{{1, 64, 80}, {0, 855, 855}, 0}, kExp64{{100, 64, 700}, {kNever, kNever, 329}, 80};
     constexpr Worth kLog32{{150, 125, 80}, {658, 658, 329}, 41}, kLog64{{300, 100, 2000}, {6000, 658, 526}, 80};
-    constexpr Worth kFmexp32{{64, 125, 500}, {526, 526, 658}, 41};
-    constexpr Worth kFmexp64{{150, 150, 700}, {329, 200, 1316}, 100};
+    constexpr Worth kFmexp32{{1, 64, 80}, {0, 395, 329}, 32}, kFmexp64{{64, 100, 700}, {kNever, 395, 329}, 80};
     if (!(g.depth == 1 && kind != IntermediateKind::Log) &&
         !worth(kind == IntermediateKind::Exp ? (fp64 ? kExp64 : kExp32)
                : kind == IntermediateKind::Log ? (fp64 ? kLog64 : kLog32)
@@ -84,9 +82,9 @@ bool column_horner_fits(const Geometry& g, const DeviceInfo& dev, IntermediateKi
                g, dev, batch))
         return false;
     const bool fm = kind == IntermediateKind::FMExp;
-    // (an exponent without degree one leaves degrees of its exponential that have no
-    // terms: the general kernel skips them, a product with their zeros would turn
-    // the multiplier's infinities into NaN)
+    // (an exponent without degree one leaves degrees of the running tensor that have
+    // no terms: the general kernel skips them, a product with their zeros would turn
+    // the exponent's infinities into NaN)
     if (fm && (x.lo > 1 || x.hi < 1)) return false;
     return out.lo <= out.hi && (fm || out.lo == 0) && horner_fits(g, dev, horner_smem<T>(g, fm));
 }

@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_colum
 }
 
 // X = alpha * L2T * lambda on degrees [lo, hi], out = exp(X) or M (x) exp(X)
-// (lie_fused.cu's k_lie_exp).  With a multiplier, W5 D5 batch 4096: FP64 778 ->
-// 531 us (66 % of the FP64 peak in these multiply-adds), FP32 422 -> 187; W3 D6
-// (3 000) FP64 226 -> 145.
+// (lie_fused.cu's k_lie_exp).  With a multiplier, W5 D5 batch 4096: FP64 777 -> 395
+// us, FP32 419 -> 150; W3 D6 (3 000) FP64 226 -> 112; rounding error against 128 bits
+// 0.6 to 0.8 of the general kernel's.
 template <typename T, int W>
 __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_column_lie_exp(Geometry G, CsrDevice mat, const T* lie,
                                                                    int64_t lie_stride, int lo, int hi, TArg<T> out,
@@ -72,8 +72,7 @@ __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_colum
         __syncthreads();
         T* o = out.at(b);
         if (fm) {
-            horner_in_place<T, W, false>(G, H, X, xlo, xhi, buf, half);
-            multiply_out<T, W>(G, o, out.lo, ohi, M, mlo, mhi, X, H);
+            horner_multiplied<T, W>(G, o, out.lo, ohi, M, mlo, mhi, Opnd<T>{X, xlo, xhi}, buf, buf + half);
         } else {
             const T unit = horner<T, W, false>(G, H, Opnd<T>{X, xlo, xhi}, buf, buf + half,
                                                [&](int n, uint32_t at, T v) { o[G.db[n] + at] = v; });
@@ -123,7 +122,7 @@ bool column_lie_exp_fits(const Geometry& g, const DeviceInfo& dev, const CsrDevi
                          bool multiplier, int lo, int hi, int64_t batch) {
     constexpr bool fp64 = std::is_same<T, double>::value;
     constexpr Worth kExp32{{150, 500, 700}, {526, 855, 1316}, 41}, kExp64{{150, 150, 700}, {0, 0, 1974}, 0};
-    constexpr Worth kFmexp32{{300, 500, 700}, {855, 1500, 1974}, 41}, kFmexp64{{1, 350, 700}, {0, 855, 2400}, 0};
+    constexpr Worth kFmexp32{{40, 500, 700}, {263, 1053, 1053}, 0}, kFmexp64{{100, 100, 700}, {0, 0, 1600}, 0};
     if (!worth(multiplier ? (fp64 ? kFmexp64 : kFmexp32) : (fp64 ? kExp64 : kExp32), g, dev, batch)) return false;
     // (an exponent without degree one: see column_horner_fits)
     if (multiplier && (lo > 1 || hi < 1)) return false;
