@@ -22,9 +22,14 @@
 // these and the index instructions are what bounds it.  Subsets -> letters (us),
 // batch 4096 unless said: st_mul FP64 W5 D5 832 -> 687, W6 D5 (2048) 1432 -> 911, W2
 // D8 652 -> 181, FP32 W5 D5 496 -> 333, W8 D4 376 -> 262; st_adj_mul FP64 W2 D8 2570 ->
-// 418, W3 D6 (3000) 661 -> 376, FP32 W5 D5 686 -> 479, W2 D8 2342 -> 161; left_hs_mul
-// FP32 W4 D3 (8192) 17.7 -> 8.9; left_hs_adj_lmul / _rmul W2 D8 FP64 1032 -> 264 / 1771
-// -> 302, FP32 935 -> 144 / 1633 -> 150.
+// 428, W3 D6 (3000) 661 -> 376, FP32 W5 D5 686 -> 479, W2 D8 2337 -> 167; left_hs_mul
+// FP32 W4 D3 (8192) 17.7 -> 8.9; left_hs_adj_lmul / _rmul W2 D8 FP64 1033 -> 274 / 1773
+// -> 312, FP32 937 -> 144 / 1632 -> 152.  What the adjoint's order costs: with whole
+// degrees in the order u v r, lanes of a sum on consecutive v and a narrow sum over
+// all warps, st_adj_mul alone took 249 at W2 D8 and 279 at W3 D6 in FP64; that order
+// has no place for the half-shuffle forms.  It is not the banks: lanes that start at
+// their own u, where W is a power of two, take 0.87 to 1.15 times as long, 1.05 in
+// most cases; nor the one first letter at a time (all of them at W3 D6 FP64: 1.12).
 #include <algorithm>
 #include <type_traits>
 
@@ -131,19 +136,58 @@ __global__ void __launch_bounds__(512) k_deal_adjoint(Geometry G, PowerDiv pd, i
                                 const T* row = E + (c * wq + v) * wk;
                                 const T* pc = Pu + (c0 + c) * wk;
                                 T d = T(0);
-                                if (in_u && in_v) {
+                                // two chains a long row, and the rows' sums in one: a chain
+                                // through all rows rounds more than the subset sums (FP32
+                                // st_adj_mul W5 D4 1.36 times, left adjoints 1.2 to 1.5; the
+                                // two chains cost 10 to 25 % of the time, and in FP64, where
+                                // only rows of 32 need them, 4 %)
+                                constexpr uint32_t split = sizeof(T) == 8 ? 32u : 8u;
+                                if (wk < split || (sizeof(T) == 4 && !in_u)) {
+                                    if (in_u && in_v) {
 #pragma unroll 4
-                                    for (uint32_t u = 0; u < wk; ++u) {
-                                        const T e = row[u];
-                                        s = fma(pc[u], e, s);
-                                        d = fma(Pv[u], e, d);
+                                        for (uint32_t u = 0; u < wk; ++u) {
+                                            const T e = row[u];
+                                            s = fma(pc[u], e, s);
+                                            d = fma(Pv[u], e, d);
+                                        }
+                                    } else if (in_u) {
+#pragma unroll 4
+                                        for (uint32_t u = 0; u < wk; ++u) s = fma(pc[u], row[u], s);
+                                    } else {
+#pragma unroll 4
+                                        for (uint32_t u = 0; u < wk; ++u) d = fma(Pv[u], row[u], d);
                                     }
-                                } else if (in_u) {
-#pragma unroll 4
-                                    for (uint32_t u = 0; u < wk; ++u) s = fma(pc[u], row[u], s);
                                 } else {
-#pragma unroll 4
-                                    for (uint32_t u = 0; u < wk; ++u) d = fma(Pv[u], row[u], d);
+                                    const uint32_t even = wk & ~1u;
+                                    T s0 = T(0), s1 = T(0), d1 = T(0);
+                                    if (in_u && in_v) {
+#pragma unroll 2
+                                        for (uint32_t u = 0; u < even; u += 2u) {
+                                            const T e = row[u], f = row[u + 1u];
+                                            s0 = fma(pc[u], e, s0);
+                                            s1 = fma(pc[u + 1u], f, s1);
+                                            d = fma(Pv[u], e, d);
+                                            d1 = fma(Pv[u + 1u], f, d1);
+                                        }
+                                    } else if (in_u) {
+#pragma unroll 2
+                                        for (uint32_t u = 0; u < even; u += 2u) {
+                                            s0 = fma(pc[u], row[u], s0);
+                                            s1 = fma(pc[u + 1u], row[u + 1u], s1);
+                                        }
+                                    } else {
+#pragma unroll 2
+                                        for (uint32_t u = 0; u < even; u += 2u) {
+                                            d = fma(Pv[u], row[u], d);
+                                            d1 = fma(Pv[u + 1u], row[u + 1u], d1);
+                                        }
+                                    }
+                                    if (even < wk) {
+                                        if (in_u) s0 = fma(pc[even], row[even], s0);
+                                        if (in_v) d = fma(Pv[even], row[even], d);
+                                    }
+                                    s += s0 + s1;
+                                    d += d1;
                                 }
                                 if (in_v) {
                                     const uint32_t at = G.db[q + 1] + (c0 + c) * wq + v;
@@ -159,13 +203,14 @@ __global__ void __launch_bounds__(512) k_deal_adjoint(Geometry G, PowerDiv pd, i
                             for (uint32_t c = 0; c < block; ++c) {
                                 const T* row = E + (c * wq + v) * wk;
                                 const T* pc = Pu + (c0 + c) * wk;
-                                T d = T(0);
+                                T d = T(0), part = T(0);
 #pragma unroll 2
                                 for (uint32_t u = lane; u < wk; u += 32u) {
                                     const T e = row[u];
-                                    if (in_u) s = fma(pc[u], e, s);
+                                    if (in_u) part = fma(pc[u], e, part);
                                     if (in_v) d = fma(Pv[u], e, d);
                                 }
+                                s += part;
                                 if (in_v) {
 #pragma unroll
                                     for (uint32_t off = 16u; off > 0u; off /= 2u) d += __shfl_down_sync(0xffffffffu, d, off);
@@ -245,9 +290,18 @@ __global__ void __launch_bounds__(512) k_deal_product(Geometry G, PowerDiv pd, i
                         v = fma(L(N, c * S + j), R(0, 0), v);
                         if (both) v = fma(L(M, j), R(1, c), v);
                     }
+                    if (M == 2) {  // k = 1, dealt here: no sum is rounded that one word alone needs
+                        const uint32_t a = j / W, e = j - a * W;
+                        v = fma(L(2, c * W + a), R(1, e), v);
+                        v = fma(L(2, c * W + e), R(1, a), v);
+                        if (both) {
+                            v = fma(L(1, a), R(2, c * W + e), v);
+                            v = fma(L(1, e), R(2, c * W + a), v);
+                        }
+                    }
                     g[i] = v;
                 }
-                for (int k = 1; k < M; ++k) {
+                for (int k = 1; k < M && M > 2; ++k) {
                     T* E = g + static_cast<uint32_t>(k) * size;
                     const T *Lc = sL + G.db[k + 1], *Lu = sL + G.db[k], *Rv = sR + G.db[M - k], *Rc = sR + G.db[M - k + 1];
                     const uint32_t wk = G.pw[k], wv = G.pw[M - k];
@@ -262,7 +316,7 @@ __global__ void __launch_bounds__(512) k_deal_product(Geometry G, PowerDiv pd, i
                     }
                 }
                 __syncthreads();
-                for (int m = M - 1; m >= 1; --m)
+                for (int m = M - 1; m >= 1 && M > 2; --m)
                     for (int k = 1; k <= m; ++k) {
                         const T* E = g + static_cast<uint32_t>(k) * size;
                         T* prev = g + static_cast<uint32_t>(k - 1) * size;  // (k = 1: the product)
@@ -364,23 +418,24 @@ int letters_need(const Geometry& g, ShuffleAdjKind kind) {
     constexpr bool fp64 = std::is_same<T, double>::value;
     const int W = g.width, D = g.depth;
     if (fp64 && D < 6) return kNone;
-    if (fp64 && W == 3 && D == 6) return kSome;
+    // (FP64 W3 D6, left: 0.79 of the subsets' time, but 1.5 times their rounding error)
+    if (fp64 && W == 3 && D == 6) return kind == ShuffleAdjKind::HalfL ? kNone : kSome;
     if (kind == ShuffleAdjKind::Shuffle) {
         if (W == 2 || D >= 6 || (W == 3 && D <= 4) || (W == 4 && D == 5)) return kAny;
         // (all first letters at once, in one long pass a degree: 1.3 times the subsets' time)
         if (W == 7 && D == 4) return kNone;
         if (D == 4 && (W == 5 || W == 6)) return kFew;
-        return D == 3 && W >= 5 && W <= 7 ? kFull : 4;
+        return D == 3 && W >= 5 && W <= 7 ? kMany : 4;
     }
     if (W >= 4 && D >= 6) return kFew;
     if (kind == ShuffleAdjKind::HalfL) {
-        if (D < 6 && g.dim > 1200) return kNone;
+        if (D < 6 && g.dim > 700) return kNone;
         if ((W == 2 && D >= 4) || (W == 3 && (D == 4 || D >= 6))) return kAny;
-        return W == 5 || W == 7 ? kMany : kFull;
+        return W >= 5 && W <= 7 ? kMany : kFull;
     }
-    if (D < 6 && (D < 4 || g.dim > 5000)) return kNone;
+    if (D < 6 && (D < 4 || W == 6 || g.dim > 5000)) return kNone;
     if ((W <= 3 && D >= 5) || W == 7) return kAny;
-    return W == 6 || (W == 2 && D == 4) ? kMany : W == 4 ? 4 : kFull;
+    return W == 2 && D == 4 ? kMany : W == 4 ? 4 : kFull;
 }
 
 template <typename T, typename Kind>
