@@ -186,17 +186,17 @@ __device__ __forceinline__ T horner(const Geometry& G, int H, const Opnd<T>& X, 
     return scaled ? c * rc.inv_fact[H] : c;  // (log: 0)
 }
 
-// The same with the whole result in X's buffer `x` (levels 0 .. H).
+// log with the whole result in X's buffer `x` (levels 0 .. H).
 // `buf`: both running buffers, `half` elements each.  Level H replaces X's,
 // which only its coefficients' own threads read; the levels below go to the
 // buffer that the last round does not read, and from there to x.  Ends with a
 // barrier.
-template <typename T, int W, bool Log>
-__device__ __forceinline__ void horner_in_place(const Geometry& G, int H, T* x, int xlo, int xhi, T* buf,
-                                                uint32_t half) {
+template <typename T, int W>
+__device__ __forceinline__ void log_in_place(const Geometry& G, int H, T* x, int xlo, int xhi, T* buf,
+                                             uint32_t half) {
     // the last round reads the buffer of its parity and may fill the other
     T* low = (H & 1) ? buf + half : buf;
-    const T unit = horner<T, W, Log>(G, H, Opnd<T>{x, xlo, xhi}, buf, buf + half, [&](int n, uint32_t at, T v) {
+    const T unit = horner<T, W, true>(G, H, Opnd<T>{x, xlo, xhi}, buf, buf + half, [&](int n, uint32_t at, T v) {
         (n == H ? x : low)[G.db[n] + at] = v;
     });
     const uint32_t below = G.db[H];

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_colum
         BulkStage<T> st(bar, phase);
         T* X = st.add(s_x, x.at(b), xlo, xhi, G);
         if (!st.commit(G.fault)) return;
-        horner_in_place<T, W, true>(G, hi, X, xlo, xhi, buf, half);
+        log_in_place<T, W>(G, hi, X, xlo, xhi, buf, half);
         sell_rows<true, true>(m, X, out + b * out_stride, out_size, alpha);  // t2l: long rows
         bulk_stage_reuse();
     }
