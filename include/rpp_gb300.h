@@ -355,7 +355,8 @@ int rpp_gb_conversion_matrix(int32_t width, int32_t depth, int32_t which, int64_
  * A call without a recorded schedule takes one chosen from the shape, the batch
  * and what it computes (CTA size, one launch or two, which arrays are kept in
  * stream-ordered workspaces); outputs of different schedules agree up to
- * rounding.
+ * rounding, so the last bits of a path's result may depend on the batch that it
+ * is computed in (pin a schedule where they must not).
  *
  * Equal-length batches too small to fill the GPU with one path per CTA are cut
  * in time where that is faster (a rule on the shape, the batch and the length,
@@ -364,6 +365,16 @@ int rpp_gb_conversion_matrix(int32_t width, int32_t depth, int32_t which, int64_
  * of at most 256 MB (the paths run whole where it cannot be had).  The results
  * are those of the whole path up to rounding, and the same for the same
  * arguments.
+ *
+ * Scratch and workspaces come from a memory pool of the library's own, one a
+ * device, which keeps at most 256 MB while the device has a plan and gives it
+ * back with the last one.  Captured in a CUDA graph they become memory nodes (a
+ * graph with memory nodes cannot be a child graph or be instantiated twice at
+ * once): a ragged batch's order, a large state's workspace, and, of equal-length
+ * calls, the pieces of paths cut in time and a default schedule's workspace.  For
+ * graphs without them, capture rpp_gb_signature_static_scratch, or
+ * rpp_gb_signature_with_schedule with a schedule that has no workspace, which
+ * never cuts a path.
  *
  * rpp_gb_signature_backward: the reverse pass alone, from final signatures
  * `sig` (as produced by rpp_gb_signature) and cotangents `seed`.
@@ -401,10 +412,11 @@ int rpp_gb_signature_host(const rpp_gb_plan* plan, rpp_gb_stream stream, int32_t
  * runtimes that own all device memory through their own allocator and forbid
  * cudaMalloc / cudaMallocAsync from plugins, real-time loops that must not wait
  * on or grow a memory pool, and hosts that budget device memory up front.
- * Same arguments and numerics as rpp_gb_signature, and the same results (up to
- * rounding where that entry cuts few long paths in time); the only scratch it
- * needs (the work counter and longest-first order of a ragged batch) lives
- * in a fixed 8 MiB device array of the library, held by every GPU that loads
+ * Same arguments and numerics as rpp_gb_signature, and the same results up to
+ * rounding (without a recorded schedule that entry picks its form by shape and
+ * batch and may cut few long paths in time, this one runs the paths whole in one
+ * launch); the only scratch it needs (the work counter and longest-first order
+ * of a ragged batch) lives in a fixed 8 MiB device array of the library, held by every GPU that loads
  * the library until the process exits.  Limits: a ragged batch of at most
  * 2,097,088 paths (RPP_GB_OUT_OF_BOUNDS beyond), and only shapes whose state
  * fits one CTA's shared memory (RPP_GB_NOT_IMPLEMENTED otherwise, e.g. width 6

@@ -35,11 +35,11 @@ __host__ __device__ inline uint32_t chen_chain_elems(const Geometry& G, int H) {
 // coefficient where the general Horner rounds multiply whole tensors D times
 // over.  One pass over memory: M is staged by one bulk copy (read as it goes
 // where that would leave one CTA an SM), the chains of two stages are kept in
-// shared memory and the result is written from the stage that forms it; HBM
-// bounds it.  ft_fmexp with increments, the general rounds -> this: FP32 W5 D5
-// batch 4096 221 -> 32 us (3.9 TB/s), W3 D6 batch 3000 89 -> 19; FP64 W5 D5
-// 455 -> 53 us (4.9 TB/s), W2 D12 batch 2048 1463 -> 117, W6 D6 batch 256
-// 1130 -> 145.
+// shared memory and the result is written from the stage that forms it.  Large
+// tensors are bound by HBM, small ones by the stages' latency.  ft_fmexp with
+// increments, the general rounds -> this: FP32 W5 D5 batch 4096 221 -> 32 us (3.9
+// TB/s), W3 D6 batch 3000 89 -> 9; FP64 W5 D5 455 -> 53 us (4.9 TB/s), W2 D12
+// batch 2048 1463 -> 117, W6 D6 batch 256 1130 -> 145.
 // Chains start at the output's lowest degree (levels of M below it take no
 // part) and degrees that M lacks count as zero, as in those rounds.
 template <typename T, int W>

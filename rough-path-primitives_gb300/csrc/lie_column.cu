@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_colum
 // X = alpha * L2T * lambda on degrees [lo, hi], out = exp(X) or M (x) exp(X)
 // (lie_fused.cu's k_lie_exp).  With a multiplier, W5 D5 batch 4096: FP64 777 -> 395
 // us, FP32 419 -> 150; W3 D6 (3 000) FP64 226 -> 112; rounding error against 128 bits
-// 0.6 to 0.8 of the general kernel's.
+// 0.6 to 0.8 of the general kernel's.  FP64 W5 D5: that pipe 71 % busy, 7.5 of 20 stalled
+// cycles an instruction on shared memory, 3.5 at barriers, three CTAs an SM.
 template <typename T, int W>
 __global__ void __launch_bounds__(kHornerThreads, (kHornerBlocks<T, W>)) k_column_lie_exp(Geometry G, CsrDevice mat, const T* lie,
                                                                    int64_t lie_stride, int lo, int hi, TArg<T> out,

@@ -33,9 +33,9 @@ cudaError_t launch_product(const Geometry& g, const DeviceInfo& dev, cudaStream_
                            TArg<T> out, TArg<T> x, TArg<T> y, TArg<T> z, int64_t batch, double alpha,
                            double beta);
 
-// The column form of launch_product (widths 2..8, both factors in
-// shared memory) and the one-pass form of exp / fmexp
-// for an exponent of degree one (ft_column.cu).
+// The column form of launch_product (widths 2..8, both factors in shared memory,
+// ft_column.cu; `added`: with a third term) and the one-pass form of exp / fmexp
+// for an exponent of degree one (ft_chen.cu).
 template <typename T>
 bool column_product_fits(const Geometry& g, const DeviceInfo& dev, bool added, int64_t batch);
 template <typename T>

@@ -213,12 +213,13 @@ cudaError_t scratch_alloc(int device, void** out, size_t bytes, cudaStream_t s) 
 // 4.0, W2 D10 6.4, W6 D5 5.8 forward, four times that with the reverse pass;
 // warp-per-letter 0.13 and 0.7 us); a call's joins cost 50 us and each round 5
 // at most (several launches of a call that is waited for), twice that with the
-// reverse pass.
+// reverse pass.  (The joins' cost was fitted to an earlier, slower form of them,
+// so calls near the line still run whole that pieces would speed up.)
 // Measured, forward + reverse, whole -> in pieces: FP64 W3 D5, 4 paths of 1 000,
-// 10.2 -> 0.24 ms; W5 D5 1 path of 1 000 16.3 -> 0.32, 100 paths 16.3 -> 5.8;
-// 64 increments, 8 paths 1.05 -> 0.23; W2 D10 FP32 1 path of 1 000 21.7 -> 0.29.
-// Where SMs are not idle pieces lose: W5 D5 FP64, 1 000 paths of 64, 3.35 ms
-// whole, 3.67 in four.
+// 10.13 -> 0.17 ms; W5 D5 1 path of 1 000 15.5 -> 0.27, 100 paths 15.6 -> 5.6;
+// 64 increments, 8 paths 1.00 -> 0.18; W2 D10 FP32 1 path of 1 000 22.0 -> 0.26.
+// Where SMs are not idle pieces lost: W5 D5 FP64, 1 000 paths of 64, 3.35 ms
+// whole, 3.67 in four (with that earlier form).
 template <typename T>
 int64_t signature_chunks(const Geometry& g, const DeviceInfo& dev, int64_t batch, int64_t length, bool reverse) {
     const int D = g.depth;
